@@ -116,7 +116,7 @@ struct md_ctx {
     // work sets (lane 0 serves every form; lane 1 the batched graph)
     int batch = 1;
     int plan = 0;   // radix plan variant of the plane top-t kernel (C2RPlan)
-    int tile = 32;  // kz lines per CTA of the x-line kernel (8, 16 or 32)
+    int tile = 32;  // md_set_tile's value: every size has one x-line shape (XPlan), so it selects nothing
     int lanes = kLanes;   // work sets / capture streams the batched graph alternates over (1 or 2)
     int cap = 0, cap_t = 0, cap_na = 0;
     WorkSet::Sizes have{};           // bytes held by each work-set buffer
@@ -182,8 +182,6 @@ struct Sized {
         else
             k_plane_fwd<N, MODE><<<dim3(NG, nb), kNT1, smem_fwd(), s>>>(L, G, vbits, qlist, qcount, sr, si, A, vr, vi);
     }
-    template <int LT = kLT>
-    static size_t smem_xline() { return xline_smem<N, LT>(); }
     template <int V = 0>
     static size_t smem_c2r() { return c2r_smem<N, V>(); }
 
@@ -218,10 +216,7 @@ struct Sized {
         set((const void *)k_xline_rec<N>, smem_xrec());
         set((const void *)k_vox_bits<NG, true>, smem_vox());
         set((const void *)k_vox_bits<NG, false>, smem_vox());
-        if constexpr (xline_tile_fits<N, 32>()) set((const void *)k_xline_herm<N, 32>, smem_xline<32>());
-        set((const void *)k_xline_herm<N, 16>, smem_xline<16>());
-        set((const void *)k_xline_herm<N, 8>, smem_xline<8>());
-        if constexpr (xline_fold_ok<N>()) set((const void *)k_xline_fold<N, 16>, smem_xline<16>());
+        set((const void *)k_xline_fold<N>, xline_smem<N>());
         if (e == cudaSuccess) done = true;
         return e;
     }
@@ -327,26 +322,7 @@ struct Sized {
         if (ev) cudaEventRecord(ev[1], s);
         any_fwd<0>(s, nb, L, G, w.vbits, w.qlist, w.qcount, nullptr, nullptr, w.A, nullptr, nullptr);
         if (ev) cudaEventRecord(ev[2], s);
-        bool folded = false;   // the register-fold form, instantiated only where it is used
-        if constexpr (xline_fold_ok<N>()) {
-            if (c->tile == 16) {
-                k_xline_fold<N, 16><<<xline_grid<N>(NH * ((N + 15) / 16), nb), 256, smem_xline<16>(), s>>>(
-                    G, w.A, c->d_Rh, w.G);
-                folded = true;
-            }
-        }
-        if (folded) {
-        } else if (c->tile == 16)
-            k_xline_herm<N, 16><<<xline_grid<N>(NH * ((N + 15) / 16), nb), 256, smem_xline<16>(), s>>>(G, w.A, c->d_Rh,
-                                                                                                      w.G);
-        else if (c->tile == 8)
-            k_xline_herm<N, 8><<<xline_grid<N>(NH * ((N + 7) / 8), nb), 128, smem_xline<8>(), s>>>(G, w.A, c->d_Rh, w.G);
-        else if constexpr (xline_tile_fits<N, 32>())
-            k_xline_herm<N, 32><<<xline_grid<N>(NH * ((N + 31) / 32), nb), 512, smem_xline<32>(), s>>>(G, w.A, c->d_Rh,
-                                                                                                      w.G);
-        else
-            k_xline_herm<N, 16><<<xline_grid<N>(NH * ((N + 15) / 16), nb), 256, smem_xline<16>(), s>>>(G, w.A, c->d_Rh,
-                                                                                                      w.G);
+        k_xline_fold<N><<<xline_grid<N>(nb), XPlan<N>::NT, xline_smem<N>(), s>>>(G, w.A, c->d_Rh, w.G);
         if (ev) cudaEventRecord(ev[3], s);
         plane_topt(s, G, w.G, nb, t, nf3f, w.cand, c->plan);
         if (ev) cudaEventRecord(ev[4], s);

@@ -848,45 +848,95 @@ __global__ void __launch_bounds__(kNT)
 // ky = 0 and ky = N/2 into row 0 (row0 = g(ky=0) + i g(ky=N/2)); both become
 // real after the inverse along kz, so the plane kernel can unpack them.
 //
-// CTA = (ky in [0, N/2), 32 kz lines).  Per pass it loads the own tile
-// (ky, kz) and the mirror tile (-ky, -kz) straight from global memory into
-// the pruned forward x-FFT, multiplies both by conj(R^), folds the mirror into
-// H and runs the inverse x-FFT of the own tile.  CTAs of row 0 run two passes
-// (ky = 0 and ky = N/2) and pack them.  Output Gh[x][ky][kz], ky < N/2.
-// LT kz lines per CTA (the tile shape the autotuner picks: 8, 16 or 32), 16 LT
-// threads, xline_occ<N>() / LT CTAs per SM (below).
+// One CTA works on tiles of LT kz lines of one row pair: the own tile (ky, kz)
+// and the mirror tile (-ky, -kz), F1 threads per line.  Forward split F1 x F2
+// (pass 1 a DFT-F1 over stride F2, straight from global memory; pass 2 a
+// DFT-F2 whose outputs sit at kx = u + F1 k2): the conjugate partner -kx of
+// every output of the own item u is an output of the mirror item (F1 - u) mod
+// F1, so one thread transforms both, multiplies both by conj(R^), folds them
+// into H in registers and runs the first inverse pass (a DFT-F2 over the same
+// stride F1, the inverse split being F2 x F1) before anything is stored: three
+// barriers per pass.  CTAs of row 0 run two passes (ky = 0 and ky = N/2) and
+// pack them.  Output Gh[x][ky][kz], ky < N/2.
 //
-// xline_occ: threads per SM the kernel is compiled for, in units of 16:
-// 1,280 where that register budget (51 per thread) holds the kernel without
-// spills, 512 above N = 160 (radices up to 20 need the registers), else 1,024.
-// B200, 13,824 rotations at 192 per launch: +2.0 % at N=96; with spills at
-// N=112 it lost 2 %.  N = 128 runs 1,280 since its first-pass loads are issued
-// ahead of the DFTs and its twiddles come from shared memory (xline_tw_smem).
+// Bound by instruction issue and the latency of the tile loads (ncu, N = 160:
+// 64 % issue active, 36 % of DRAM peak; N = 256: 41 % and 33 %), so a plan
+// trades radix against warps: F1 near 2 F2 keeps the registers of both passes
+// level, F1 threads per line leave none idle in the two larger passes, and LT
+// = 8 above N = 196 keeps three or more CTAs per SM.  A form that stored the
+// mirror products to shared memory and folded in a pass of its own (five
+// barriers, 16 threads per line) took, against this one, in us per rotation
+// (B200, random planes, 5 to 128 rotations per launch): N = 60 1.25 -> 0.63,
+// 96 2.33 -> 2.06, 108 4.80 -> 3.49, 126 7.6 -> 5.8, 144 8.4 -> 6.7, 160 12.2
+// -> 10.5, 180 54 -> 20, 216 93 -> 32, 250 133 -> 56, 330 198 -> 139 (above
+// 160 half of that from the block order, xline_rot_fast).
+//
+// MDB_XPLAN(N, F1, F2, LT, CTAs per SM, SEQ): the fastest measured among the
+// splits, at the residencies their registers allow.  SEQ finishes the own
+// item's product before it reads the mirror item: without it a radix-16 item
+// pair runs out of registers (N = 256 54 -> 47, the older form 50; N = 320 121
+// -> 112; slower by up to 9 % elsewhere).  Four sizes lost to the older form's
+// shorter items (N = 336 136 -> 145, 352 157 -> 173, 384 187 -> 218, 432 364
+// -> 372); every other one gained.
 template <int N>
-constexpr int xline_occ() {
-    return (N == 32 || N == 64 || N == 72 || N == 80 || N == 96 || N == 128) ? 80 : (N > 160 ? 32 : 64);
-}
+struct XPlan;
+#define MDB_XPLAN(N_, F1_, F2_, LT_, OCC_, SEQ_)                               \
+    template <>                                                                 \
+    struct XPlan<N_> {                                                          \
+        static constexpr int F1 = F1_, F2 = F2_, LT = LT_, OCC = OCC_;          \
+        static constexpr bool SEQ = SEQ_;                                       \
+        static constexpr int NT = F1 * LT, TILES = (N_ + LT - 1) / LT;          \
+        static_assert(F1_ * F2_ == N_ && NT <= 1024, "plan");                   \
+    };
+MDB_XPLAN(32, 8, 4, 16, 8, 0) MDB_XPLAN(36, 6, 6, 16, 8, 0) MDB_XPLAN(40, 10, 4, 16, 6, 0)
+MDB_XPLAN(42, 6, 7, 16, 10, 0) MDB_XPLAN(44, 11, 4, 16, 6, 0) MDB_XPLAN(48, 8, 6, 16, 8, 0)
+MDB_XPLAN(50, 10, 5, 16, 7, 0) MDB_XPLAN(54, 9, 6, 16, 6, 0) MDB_XPLAN(56, 8, 7, 16, 8, 0)
+MDB_XPLAN(60, 12, 5, 16, 6, 0) MDB_XPLAN(64, 8, 8, 16, 7, 0) MDB_XPLAN(66, 11, 6, 16, 6, 0)
+MDB_XPLAN(70, 14, 5, 16, 5, 0) MDB_XPLAN(72, 12, 6, 16, 5, 0) MDB_XPLAN(80, 10, 8, 16, 6, 0)
+MDB_XPLAN(84, 14, 6, 16, 5, 0) MDB_XPLAN(88, 11, 8, 16, 5, 0) MDB_XPLAN(90, 15, 6, 16, 4, 0)
+MDB_XPLAN(96, 12, 8, 16, 5, 0) MDB_XPLAN(98, 14, 7, 16, 4, 0) MDB_XPLAN(100, 10, 10, 16, 4, 0)
+MDB_XPLAN(108, 18, 6, 16, 4, 0) MDB_XPLAN(110, 10, 11, 16, 4, 0) MDB_XPLAN(112, 16, 7, 16, 4, 0)
+MDB_XPLAN(120, 15, 8, 16, 4, 0) MDB_XPLAN(126, 14, 9, 16, 4, 0) MDB_XPLAN(128, 16, 8, 16, 4, 0)
+MDB_XPLAN(132, 12, 11, 16, 4, 0) MDB_XPLAN(140, 20, 7, 16, 3, 0) MDB_XPLAN(144, 12, 12, 16, 4, 0)
+MDB_XPLAN(150, 15, 10, 16, 4, 0) MDB_XPLAN(154, 14, 11, 16, 3, 0) MDB_XPLAN(160, 20, 8, 16, 3, 0)
+MDB_XPLAN(162, 18, 9, 16, 3, 0) MDB_XPLAN(168, 24, 7, 16, 2, 0) MDB_XPLAN(176, 16, 11, 16, 3, 0)
+MDB_XPLAN(180, 20, 9, 16, 3, 0) MDB_XPLAN(192, 24, 8, 16, 3, 0) MDB_XPLAN(196, 28, 7, 16, 2, 0)
+MDB_XPLAN(198, 22, 9, 16, 2, 0) MDB_XPLAN(200, 20, 10, 8, 6, 0) MDB_XPLAN(210, 21, 10, 8, 4, 0)
+MDB_XPLAN(216, 24, 9, 8, 4, 0) MDB_XPLAN(220, 20, 11, 8, 4, 0) MDB_XPLAN(224, 28, 8, 16, 2, 0)
+MDB_XPLAN(240, 24, 10, 16, 2, 0) MDB_XPLAN(242, 22, 11, 8, 4, 0) MDB_XPLAN(250, 25, 10, 8, 4, 0)
+MDB_XPLAN(252, 28, 9, 8, 4, 0) MDB_XPLAN(256, 16, 16, 16, 2, 1) MDB_XPLAN(264, 24, 11, 16, 2, 0)
+MDB_XPLAN(270, 27, 10, 8, 4, 0) MDB_XPLAN(280, 28, 10, 8, 4, 0) MDB_XPLAN(288, 24, 12, 8, 4, 0)
+MDB_XPLAN(294, 21, 14, 8, 4, 0) MDB_XPLAN(300, 30, 10, 8, 3, 0) MDB_XPLAN(308, 28, 11, 8, 3, 0)
+MDB_XPLAN(320, 32, 10, 8, 3, 1) MDB_XPLAN(324, 36, 9, 8, 2, 0) MDB_XPLAN(330, 30, 11, 8, 3, 0)
+MDB_XPLAN(336, 28, 12, 8, 3, 0) MDB_XPLAN(350, 35, 10, 8, 2, 0) MDB_XPLAN(352, 32, 11, 8, 2, 0)
+MDB_XPLAN(360, 30, 12, 8, 3, 0) MDB_XPLAN(378, 27, 14, 8, 3, 0) MDB_XPLAN(384, 32, 12, 8, 3, 0)
+MDB_XPLAN(392, 28, 14, 8, 3, 0) MDB_XPLAN(396, 36, 11, 8, 2, 0) MDB_XPLAN(400, 20, 20, 8, 3, 0)
+MDB_XPLAN(420, 35, 12, 8, 2, 0) MDB_XPLAN(432, 36, 12, 8, 2, 0) MDB_XPLAN(440, 40, 11, 8, 2, 0)
+MDB_XPLAN(448, 32, 14, 8, 3, 0) MDB_XPLAN(450, 30, 15, 8, 2, 0) MDB_XPLAN(462, 33, 14, 8, 2, 0)
+MDB_XPLAN(480, 40, 12, 8, 2, 0) MDB_XPLAN(484, 44, 11, 8, 2, 0) MDB_XPLAN(486, 27, 18, 8, 3, 0)
+MDB_XPLAN(490, 35, 14, 8, 2, 0) MDB_XPLAN(500, 50, 10, 8, 2, 0) MDB_XPLAN(504, 36, 14, 8, 2, 0)
+MDB_XPLAN(512, 32, 16, 8, 2, 1)
+#undef MDB_XPLAN
 
-// Twiddles of the x-line kernel from shared memory instead of the read-only
-// cache.  Measured at N = 128 (B200, 54,000 rotations, 192 per launch): with
-// five 256-thread CTAs per SM (48 registers) 267 ms per step for this kernel,
-// against 277 ms with cached loads and 278 ms at four CTAs per SM; at four
-// CTAs per SM the shared-memory table lost (285 ms).  Other sizes keep the
-// cached loads.
+// Twiddles from a shared-memory table instead of the read-only cache, and tile
+// addresses formed per access instead of from a running pointer: N = 128,
+// whose register budget (64 at four CTAs per SM) the pointer form exceeds
+// (4.41 us per rotation against 6.9 with 176 bytes of spills).
 template <int N>
 constexpr bool xline_tw_smem() {
     return N == 128;
 }
 
-// Block order of the x-line kernels.  Every launch-group rotation reads the
-// same receptor spectrum tiles, which stay in L2 across the launch while the
-// spectrum fits (16 MiB at N = 128); above N = 224 it does not (8 N^3 bytes,
-// 134 MB at N = 256), so the rotation becomes the fastest-varying block index
-// and the launch's rotations read each (ky, kz-tile) of R^ back to back from
-// L2 instead of streaming all of it from HBM once per rotation.
+// Block order.  Every launch-group rotation reads the same receptor spectrum
+// tiles.  Up to N = 144 the spectrum (8 N^3 bytes, 24 MB) stays in L2 beside
+// the streamed planes, and neighbouring tiles run together; above, the
+// rotation is the fastest-varying block index, so the launch's rotations read
+// each (ky, kz-tile) of R^ back to back from L2 instead of streaming all of it
+// from HBM once per rotation.  B200, 16-line tiles: N = 128 4.4 us per rotation
+// tile-fast, 6.9 rotation-fast; N = 160 equal within 5 %; N = 180 54 against 20.
 template <int N>
 constexpr bool xline_rot_fast() {
-    return N > 224;
+    return N > 144;
 }
 template <int N>
 __device__ __forceinline__ void xline_block(int &tile_id, int &b) {
@@ -899,207 +949,25 @@ __device__ __forceinline__ void xline_block(int &tile_id, int &b) {
     }
 }
 template <int N>
-inline dim3 xline_grid(int tiles, int nb) {
+inline dim3 xline_grid(int nb) {
+    constexpr int tiles = N / 2 * XPlan<N>::TILES;
     return xline_rot_fast<N>() ? dim3(nb, tiles) : dim3(tiles, nb);
 }
 
-// Shared memory of k_xline_herm: the own and mirror tiles, and the twiddle
-// table where xline_tw_smem<N>().
-template <int N, int LT>
+// Shared memory: the own and mirror tiles, and the twiddle table where
+// xline_tw_smem<N>().
+template <int N>
 constexpr size_t xline_smem() {
-    return (size_t)(2 * N * LT + (xline_tw_smem<N>() ? N : 0)) * sizeof(float2);
-}
-// Whether an LT-line tile fits one CTA's 227 KB (32-line tiles stop at N = 450;
-// above, a request for them runs 16-line tiles).
-template <int N, int LT>
-constexpr bool xline_tile_fits() {
-    return xline_smem<N, LT>() <= 227 * 1024;
+    return (size_t)(2 * N * XPlan<N>::LT + (xline_tw_smem<N>() ? N : 0)) * sizeof(float2);
 }
 
-template <int N, int LT = kLT>
-__global__ void __launch_bounds__(16 * LT, xline_occ<N>() / LT)
-    k_xline_herm(GridView G, const float2 *__restrict__ A, const float2 *__restrict__ Rh, float2 *__restrict__ Gh) {
-    constexpr int NG = N / 2, NH = N / 2, OFF = N / 4;
-    constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
-    constexpr bool PR = prune_ok<N>();
-    constexpr int TILES = (N + LT - 1) / LT;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2 *X0 = reinterpret_cast<float2 *>(smem_raw);   // own tile   [N][LT]
-    float2 *X1 = X0 + N * LT;                           // mirror tile [N][LT]
-    constexpr int NT = 16 * LT;
-    float2 *TWs = X1 + N * LT;                          // twiddles W_N^j (xline_tw_smem)
-    if constexpr (xline_tw_smem<N>()) {
-        for (int e = threadIdx.x; e < N; e += NT) TWs[e] = __ldg(&G.tw[e]);
-        __syncthreads();
-    }
-    auto tw_at = [&](int j) {
-        if constexpr (xline_tw_smem<N>()) return TWs[j];
-        else return __ldg(&G.tw[j]);
-    };
-    const int lane = threadIdx.x % LT;
-    int tile_id, b;
-    xline_block<N>(tile_id, b);
-    const int ky = tile_id / TILES;
-    const int kz = (tile_id % TILES) * LT + lane;
-    const bool ok = kz < N;
-    const int kzm = (N - kz) % N;
-    const float2 *Ab = A + (size_t)b * NG * N * N;
-    float2 *Gb = Gh + (size_t)b * N * NH * N;
-    const int passes = (ky == 0) ? 2 : 1;
-
-    for (int pass = 0; pass < passes; ++pass) {
-        const int kyo = pass == 0 ? ky : NH;   // own row
-        const int kym = (N - kyo) % N;         // mirror row
-        // forward x pass 1 on both tiles, straight from global (pruned rows):
-        // every item of this thread issues its loads before the first DFT, so
-        // the HBM latency is paid once per thread, not once per item
-        constexpr int IT1 = (2 * LT * R2 + NT - 1) / NT;
-        float2 v1[IT1][R1];
-#pragma unroll
-        for (int r = 0; r < IT1; ++r) {
-            const int it = threadIdx.x + r * NT;
-            const int s = it / (LT * R2);
-            const int t = (it / LT) % R2;
-            const int row = s ? kym : kyo, col = s ? kzm : kz;
-            const bool live = ok && it < 2 * LT * R2;
-            static_for<0, R1>([&](auto m_) {
-                constexpr int mm = decltype(m_)::value;
-                const int pp = t + R2 * mm - OFF;   // spectrum plane of x = t + R2 mm, if any
-                if constexpr (PR && (mm < R1 / 4 || mm >= 3 * R1 / 4)) {
-                    v1[r][mm] = make_float2(-0.f, -0.f);
-                } else if constexpr (PR) {
-                    v1[r][mm] = live ? Ab[((size_t)pp * N + row) * N + col] : make_float2(0.f, 0.f);
-                } else {
-                    v1[r][mm] = (live && (unsigned)pp < (unsigned)NG) ? Ab[((size_t)pp * N + row) * N + col]
-                                                                     : make_float2(0.f, 0.f);
-                }
-            });
-        }
-#pragma unroll
-        for (int r = 0; r < IT1; ++r) {
-            const int it = threadIdx.x + r * NT;
-            if (it < 2 * LT * R2) {
-                const int s = it / (LT * R2);
-                const int t = (it / LT) % R2;
-                Dft<R1, -1>::run(v1[r]);
-                float2 *X = s ? X1 : X0;
-                static_for<0, R1>([&](auto k1_) {
-                    constexpr int k1 = decltype(k1_)::value;
-                    float2 x = v1[r][k1];
-                    if constexpr (k1 != 0) x = cmul(x, tw_at(t * k1));
-                    X[(k1 * R2 + t) * LT + lane] = x;
-                });
-            }
-        }
-        __syncthreads();
-        // forward x pass 2 and the conj(R^) product, held in registers
-        constexpr int IPT = (2 * LT * R1 + NT - 1) / NT;
-        float2 reg[IPT][R2];
-#pragma unroll
-        for (int r = 0; r < IPT; ++r) {
-            const int it = threadIdx.x + r * NT;
-            if (it < 2 * LT * R1) {
-                const int s = it / (LT * R1);
-                const int u = (it / LT) % R1;
-                const int row = s ? kym : kyo, col = s ? kzm : kz;
-                fft_phase2<N, -1>((s ? X1 : X0) + lane, LT, u, reg[r]);
-                static_for<0, R2>([&](auto k2) {
-                    const int kx = u + R1 * k2;
-                    const float2 rh = ok ? __ldg(&Rh[((size_t)kx * N + row) * N + col]) : make_float2(0.f, 0.f);
-                    reg[r][k2] = cmulconj(rh, reg[r][k2]);
-                });
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < IPT; ++r) {
-            const int it = threadIdx.x + r * NT;
-            if (it < 2 * LT * R1) {
-                const int s = it / (LT * R1);
-                const int u = (it / LT) % R1;
-                float2 *X = s ? X1 : X0;
-                static_for<0, R2>([&](auto k2) { X[(u + R1 * k2) * LT + lane] = reg[r][k2]; });
-            }
-        }
-        __syncthreads();
-        // inverse x pass 1 of H = (P_own(kx) + conj(P_mirror(-kx))) / 2, in place in X0
-        for (int it = threadIdx.x; it < LT * R2; it += blockDim.x) {
-            const int t = it / LT;
-            float2 v[R1];
-            static_for<0, R1>([&](auto m_) {
-                constexpr int mm = decltype(m_)::value;
-                const int e = t + R2 * mm;
-                const float2 a = X0[e * LT + lane];
-                const float2 c = X1[((N - e) % N) * LT + lane];
-                v[mm] = make_float2(0.5f * (a.x + c.x), 0.5f * (a.y - c.y));
-            });
-            Dft<R1, +1>::run(v);
-            static_for<0, R1>([&](auto k1_) {
-                constexpr int k1 = decltype(k1_)::value;
-                float2 x = v[k1];
-                if constexpr (k1 != 0) x = cmul(x, conjf2(tw_at(t * k1)));
-                X0[(k1 * R2 + t) * LT + lane] = x;
-            });
-        }
-        __syncthreads();
-        // inverse x pass 2 -> Gh (row 0 packs ky = 0 and ky = N/2)
-        for (int it = threadIdx.x; it < LT * R1; it += blockDim.x) {
-            const int u = it / LT;
-            float2 o[R2];
-            fft_phase2<N, +1>(X0 + lane, LT, u, o);
-            if (ok) {
-                static_for<0, R2>([&](auto k2) {
-                    const int x = u + R1 * k2;
-                    float2 *dst = &Gb[((size_t)x * NH + ky) * N + kz];
-                    if (ky != 0 || pass == 0) {
-                        *dst = o[k2];
-                    } else {
-                        // same thread wrote the ky = 0 value in pass 0
-                        const float2 g0 = *dst;
-                        *dst = make_float2(g0.x - o[k2].y, g0.y + o[k2].x);
-                    }
-                });
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// K2, register-fold form.  The same transform as k_xline_herm with the
-// forward split reversed (pass 1 a DFT-F1 over stride F2, pass 2 a DFT-F2
-// whose outputs sit at kx = u + F1 k2): the conjugate partner -kx of every
-// output of the own item u is an output of the mirror item (F1 - u) mod F1,
-// so one thread transforms both, multiplies both by conj(R^), folds them into
-// H in registers, and runs the first inverse pass (a DFT-F2 over the same
-// stride F1, the inverse split being F2 x F1) before anything is stored.  The
-// mirror tile's products never go back to shared memory, and the fold and
-// the first inverse pass need no barrier of their own: three barriers per
-// pass instead of five.
 template <int N>
-struct FoldPlan {
-    static constexpr int F1 = Plan<N>::R2, F2 = Plan<N>::R1;
-};
-// Used for the 16-line tiles at N = 128, compiled for four 256-thread CTAs
-// per SM (64 registers).  B200, 13,824 of the 54,000 rotations at 512 per
-// launch: 237.4 ms per 54,000 rotations against 262.8 for k_xline_herm; at
-// five CTAs per SM (48 registers, 100 bytes of spills) 284.0, at three 267.2.
-template <int N>
-constexpr bool xline_fold_ok() {
-    return N == 128;
-}
-template <int N>
-constexpr int xline_fold_occ() {
-    return 64;
-}
-
-template <int N, int LT = kLT>
-__global__ void __launch_bounds__(16 * LT, xline_fold_occ<N>() / LT)
+__global__ void __launch_bounds__(XPlan<N>::NT, XPlan<N>::OCC)
     k_xline_fold(GridView G, const float2 *__restrict__ A, const float2 *__restrict__ Rh, float2 *__restrict__ Gh) {
     constexpr int NG = N / 2, NH = N / 2, OFF = N / 4;
-    constexpr int F1 = FoldPlan<N>::F1, F2 = FoldPlan<N>::F2;
-    constexpr bool PR = N % 4 == 0 && F1 % 4 == 0;
-    constexpr int TILES = (N + LT - 1) / LT;
-    constexpr int NT = 16 * LT;
+    constexpr int F1 = XPlan<N>::F1, F2 = XPlan<N>::F2, LT = XPlan<N>::LT, NT = XPlan<N>::NT;
+    constexpr int TILES = XPlan<N>::TILES;
+    constexpr bool PTR = !xline_tw_smem<N>();   // running pointers
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *X0 = reinterpret_cast<float2 *>(smem_raw);   // own tile   [N][LT]
     float2 *X1 = X0 + N * LT;                           // mirror tile [N][LT]
@@ -1117,7 +985,7 @@ __global__ void __launch_bounds__(16 * LT, xline_fold_occ<N>() / LT)
     xline_block<N>(tile_id, b);
     const int ky = tile_id / TILES;
     const int kz = (tile_id % TILES) * LT + lane;
-    const bool ok = kz < N;
+    const bool ok = N % LT == 0 || kz < N;
     const int kzm = (N - kz) % N;
     const float2 *Ab = A + (size_t)b * NG * N * N;
     float2 *Gb = Gh + (size_t)b * N * NH * N;
@@ -1127,7 +995,7 @@ __global__ void __launch_bounds__(16 * LT, xline_fold_occ<N>() / LT)
         const int kyo = pass == 0 ? ky : NH;   // own row
         const int kym = (N - kyo) % N;         // mirror row
         // forward pass 1 (DFT-F1 over stride F2) on both tiles, straight from
-        // global (pruned rows), every load of a thread issued before its DFTs
+        // global (padding pruned), every load of a thread issued before its DFTs
         constexpr int IT1 = (2 * LT * F2 + NT - 1) / NT;
         float2 v1[IT1][F1];
 #pragma unroll
@@ -1137,23 +1005,24 @@ __global__ void __launch_bounds__(16 * LT, xline_fold_occ<N>() / LT)
             const int t = (it / LT) % F2;
             const int row = s ? kym : kyo, col = s ? kzm : kz;
             const bool live = ok && it < 2 * LT * F2;
+            const float2 *src = Ab + (size_t)row * N + col + (ptrdiff_t)(t - OFF) * N * N;
             static_for<0, F1>([&](auto m_) {
                 constexpr int mm = decltype(m_)::value;
+                constexpr int st = pad_state<N, F2>(mm);
                 const int pp = t + F2 * mm - OFF;   // spectrum plane of x = t + F2 mm, if any
-                if constexpr (PR && (mm < F1 / 4 || mm >= 3 * F1 / 4)) {
+                if constexpr (st == 0) {
                     v1[r][mm] = make_float2(-0.f, -0.f);
-                } else if constexpr (PR) {
-                    v1[r][mm] = live ? Ab[((size_t)pp * N + row) * N + col] : make_float2(0.f, 0.f);
                 } else {
-                    v1[r][mm] = (live && (unsigned)pp < (unsigned)NG) ? Ab[((size_t)pp * N + row) * N + col]
-                                                                     : make_float2(0.f, 0.f);
+                    const bool in = live && (st == 2 || (unsigned)pp < (unsigned)NG);
+                    if constexpr (PTR) v1[r][mm] = in ? src[(size_t)(F2 * mm) * N * N] : make_float2(0.f, 0.f);
+                    else v1[r][mm] = in ? Ab[((size_t)pp * N + row) * N + col] : make_float2(0.f, 0.f);
                 }
             });
         }
 #pragma unroll
         for (int r = 0; r < IT1; ++r) {
             const int it = threadIdx.x + r * NT;
-            if (it < 2 * LT * F2) {
+            if ((2 * LT * F2) % NT == 0 || it < 2 * LT * F2) {
                 const int s = it / (LT * F2);
                 const int t = (it / LT) % F2;
                 Dft<F1, -1>::run(v1[r]);
@@ -1169,59 +1038,65 @@ __global__ void __launch_bounds__(16 * LT, xline_fold_occ<N>() / LT)
         __syncthreads();
         // forward pass 2 of the own item u and the mirror item (F1 - u) mod F1,
         // conj(R^) products, H = (P_own(kx) + conj P_mirror(-kx)) / 2 and the
-        // first inverse pass, in registers
-        constexpr int IT2 = (LT * F1 + NT - 1) / NT;
-        float2 h[IT2][F2];
-#pragma unroll
-        for (int r = 0; r < IT2; ++r) {
-            const int it = threadIdx.x + r * NT;
-            if (it < LT * F1) {
-                const int u = it / LT;
-                const int um = (F1 - u) % F1;
-                float2 pm[F2];
-                static_for<0, F2>([&](auto n2_) {
-                    constexpr int n2 = decltype(n2_)::value;
-                    h[r][n2] = X0[(u * F2 + n2) * LT + lane];
+        // first inverse pass, in registers (one item per thread)
+        const int u = threadIdx.x / LT;
+        const int um = (F1 - u) % F1;
+        float2 h[F2];
+        {
+            float2 pm[F2];
+            const float2 *ro = Rh + ((size_t)u * N + kyo) * N + kz, *rm = Rh + ((size_t)um * N + kym) * N + kzm;
+            auto r_own = [&](int k2) {
+                if (!ok) return make_float2(0.f, 0.f);
+                if constexpr (PTR) return __ldg(ro + (size_t)(F1 * k2) * N * N);
+                else return __ldg(&Rh[((size_t)(u + F1 * k2) * N + kyo) * N + kz]);
+            };
+            auto r_mirror = [&](int k2) {
+                if (!ok) return make_float2(0.f, 0.f);
+                if constexpr (PTR) return __ldg(rm + (size_t)(F1 * k2) * N * N);
+                else return __ldg(&Rh[((size_t)(um + F1 * k2) * N + kym) * N + kzm]);
+            };
+            if constexpr (XPlan<N>::SEQ) {
+                static_for<0, F2>([&](auto n2) { h[n2] = X0[(u * F2 + n2) * LT + lane]; });
+                Dft<F2, -1>::run(h);
+                static_for<0, F2>([&](auto k2) { h[k2] = cmulconj(r_own(k2), h[k2]); });
+                asm volatile("" ::: "memory");   // the mirror item's loads stay below
+                static_for<0, F2>([&](auto n2) { pm[n2] = X1[(um * F2 + n2) * LT + lane]; });
+                Dft<F2, -1>::run(pm);
+                static_for<0, F2>([&](auto k2) { pm[k2] = cmulconj(r_mirror(k2), pm[k2]); });
+            } else {
+                static_for<0, F2>([&](auto n2) {
+                    h[n2] = X0[(u * F2 + n2) * LT + lane];
                     pm[n2] = X1[(um * F2 + n2) * LT + lane];
                 });
-                Dft<F2, -1>::run(h[r]);
+                Dft<F2, -1>::run(h);
                 Dft<F2, -1>::run(pm);
-                static_for<0, F2>([&](auto k2_) {
-                    constexpr int k2 = decltype(k2_)::value;
-                    const float2 rov = ok ? __ldg(&Rh[((size_t)(u + F1 * k2) * N + kyo) * N + kz]) : make_float2(0.f, 0.f);
-                    const float2 rm = ok ? __ldg(&Rh[((size_t)(um + F1 * k2) * N + kym) * N + kzm]) : make_float2(0.f, 0.f);
-                    h[r][k2] = cmulconj(rov, h[r][k2]);
-                    pm[k2] = cmulconj(rm, pm[k2]);
-                });
-                // the partner of kx = u + F1 k2 is mirror output (F2 - 1 - k2)
-                // for u > 0 and (F2 - k2) mod F2 for u = 0
-                if (u == 0) {
-                    static_for<0, F2>([&](auto k2_) {
-                        constexpr int k2 = decltype(k2_)::value, j2 = (F2 - k2) % F2;
-                        h[r][k2] = make_float2(0.5f * (h[r][k2].x + pm[j2].x), 0.5f * (h[r][k2].y - pm[j2].y));
-                    });
-                } else {
-                    static_for<0, F2>([&](auto k2_) {
-                        constexpr int k2 = decltype(k2_)::value, j2 = F2 - 1 - k2;
-                        h[r][k2] = make_float2(0.5f * (h[r][k2].x + pm[j2].x), 0.5f * (h[r][k2].y - pm[j2].y));
-                    });
-                }
-                Dft<F2, +1>::run(h[r]);
-                static_for<1, F2>([&](auto k1_) {
-                    constexpr int k1 = decltype(k1_)::value;
-                    h[r][k1] = cmul(h[r][k1], conjf2(tw_at(u * k1)));
+                static_for<0, F2>([&](auto k2) {
+                    const float2 a = r_own(k2), c = r_mirror(k2);
+                    h[k2] = cmulconj(a, h[k2]);
+                    pm[k2] = cmulconj(c, pm[k2]);
                 });
             }
+            // the partner of kx = u + F1 k2 is mirror output (F2 - 1 - k2)
+            // for u > 0 and (F2 - k2) mod F2 for u = 0
+            if (u == 0) {
+                static_for<0, F2>([&](auto k2_) {
+                    constexpr int k2 = decltype(k2_)::value, j2 = (F2 - k2) % F2;
+                    h[k2] = make_float2(0.5f * (h[k2].x + pm[j2].x), 0.5f * (h[k2].y - pm[j2].y));
+                });
+            } else {
+                static_for<0, F2>([&](auto k2_) {
+                    constexpr int k2 = decltype(k2_)::value, j2 = F2 - 1 - k2;
+                    h[k2] = make_float2(0.5f * (h[k2].x + pm[j2].x), 0.5f * (h[k2].y - pm[j2].y));
+                });
+            }
+            Dft<F2, +1>::run(h);
+            static_for<1, F2>([&](auto k1_) {
+                constexpr int k1 = decltype(k1_)::value;
+                h[k1] = cmul(h[k1], conjf2(tw_at(u * k1)));
+            });
         }
         __syncthreads();
-#pragma unroll
-        for (int r = 0; r < IT2; ++r) {
-            const int it = threadIdx.x + r * NT;
-            if (it < LT * F1) {
-                const int u = it / LT;
-                static_for<0, F2>([&](auto k1) { X0[(k1 * F1 + u) * LT + lane] = h[r][k1]; });
-            }
-        }
+        static_for<0, F2>([&](auto k1) { X0[(k1 * F1 + u) * LT + lane] = h[k1]; });
         __syncthreads();
         // inverse pass 2 (DFT-F1 over items u2 < F2) -> Gh (row 0 packs ky = 0 and ky = N/2)
         for (int it = threadIdx.x; it < LT * F2; it += NT) {
@@ -1230,9 +1105,10 @@ __global__ void __launch_bounds__(16 * LT, xline_fold_occ<N>() / LT)
             static_for<0, F1>([&](auto n2) { o[decltype(n2)::value] = X0[(u2 * F1 + decltype(n2)::value) * LT + lane]; });
             Dft<F1, +1>::run(o);
             if (ok) {
+                float2 *dst0 = Gb + ((size_t)u2 * NH + ky) * N + kz;
                 static_for<0, F1>([&](auto k2) {
-                    const int x = u2 + F2 * k2;
-                    float2 *dst = &Gb[((size_t)x * NH + ky) * N + kz];
+                    float2 *dst = PTR ? dst0 + (size_t)(F2 * k2) * NH * N
+                                      : &Gb[((size_t)(u2 + F2 * k2) * NH + ky) * N + kz];
                     if (ky != 0 || pass == 0) {
                         *dst = o[k2];
                     } else {
@@ -1360,7 +1236,7 @@ struct TopList {
 };
 
 // K3: one x-plane of one rotation.  Input Gh[x][ky < N/2][kz] from
-// k_xline_herm.  (1) inverse FFT along kz of the N/2 rows, straight from
+// k_xline_fold.  (1) inverse FFT along kz of the N/2 rows, straight from
 // global memory; row 0 then holds h0 + i h_{N/2}, both real.  (2) complex-to-
 // real inverse along ky for every z column: with X the half spectrum,
 //   Z[k] = (X[k] + conj X[N/2-k]) + i w^k (X[k] - conj X[N/2-k]),  w = e^{2 pi i/N},

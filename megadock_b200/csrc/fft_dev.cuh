@@ -360,6 +360,33 @@ constexpr bool prune_ok() {
     return N % 4 == 0 && Plan<N>::R1 % 4 == 0;
 }
 
+// Zero padding of input m of a radix-R1 first pass over stride R2 on an axis
+// of length N (data in [floor(N/4), floor(N/4) + N/2)): 0 = padding for every
+// item t < R2, 2 = data for every item, 1 = depends on the item.  With
+// N % 4 == 0 and R1 % 4 == 0 no input is mixed; other splits have at most two
+// mixed inputs, so they prune as well.
+template <int N, int R2>
+constexpr int pad_state(int m) {
+    constexpr int OFF = N / 4, NG = N / 2;
+    const int lo = R2 * m, hi = R2 * m + R2 - 1;
+    if (hi < OFF || lo >= OFF + NG) return 0;
+    return (lo >= OFF && hi < OFF + NG) ? 2 : 1;
+}
+
+// The inputs of item t of a pruned first pass: load(y) reads data element
+// y in [0, N/2) (axis position y + floor(N/4)).
+template <int N, int R1, int R2, class Load>
+__device__ __forceinline__ void padded_inputs(float2 (&v)[R1], int t, const Load &load) {
+    static_for<0, R1>([&](auto m_) {
+        constexpr int m = decltype(m_)::value;
+        constexpr int st = pad_state<N, R2>(m);
+        const int y = t + R2 * m - N / 4;
+        if constexpr (st == 0) v[m] = make_float2(-0.f, -0.f);
+        else if constexpr (st == 2) v[m] = load(y);
+        else v[m] = (unsigned)y < (unsigned)(N / 2) ? load(y) : make_float2(0.f, 0.f);
+    });
+}
+
 // Phase 1 of one item on a line at `b` with element stride `es`.
 // tw: W_N^j = exp(-2*pi*i*j/N), j < N (forward table); S selects the sign.
 template <int N, int S, bool PRUNE>

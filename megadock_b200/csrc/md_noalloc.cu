@@ -78,7 +78,7 @@ int tw_offset(int n) {
 template <int N>
 struct Smem {
     static size_t fwd() { return (size_t)N * (N + 1) * sizeof(float2); }
-    static size_t xline() { return xline_smem<N, kLT>(); }
+    static size_t xline() { return xline_smem<N>(); }
     static size_t c2r() { return c2r_smem<N, 0>(); }
 };
 
@@ -89,7 +89,7 @@ cudaError_t set_attrs() {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
     set((const void *)k_plane_fwd<N, 0>, Smem<N>::fwd());
-    set((const void *)k_xline_herm<N, kLT>, Smem<N>::xline());
+    set((const void *)k_xline_fold<N>, Smem<N>::xline());
     set((const void *)k_plane_c2r<N, 1>, Smem<N>::c2r());
     set((const void *)k_plane_c2r<N, 4>, Smem<N>::c2r());
     set((const void *)k_plane_c2r<N, 16>, Smem<N>::c2r());
@@ -148,14 +148,14 @@ template <int N>
 void run_rotation(cudaStream_t s, const LigandView &L, const GridView &G, const float *rot9, const float2 *Rh,
                   const Prep &pr, uint32_t *vbits, int2 *qlist, int *qcount, float2 *A, float2 *Gsp, Cand *cand,
                   int rot, int t, DevPose *pose) {
-    constexpr int NG = N / 2, NH = N / 2, TILES = (N + kLT - 1) / kLT;
+    constexpr int NG = N / 2;
     const float nf3f = (float)((long long)N * N * N);
     k_atom_prep<NG><<<1, kNTP, 0, s>>>(L, G, rot9, pr.srec, pr.sstart, pr.cq, pr.cstart);
     k_vox_bits<NG><<<dim3(NG, 1), kNT0, vox_bits_smem<NG>(), s>>>(L, G, pr.srec, pr.sstart, pr.cq, pr.cstart, vbits,
                                                                  qlist, qcount);
     k_plane_fwd<N, 0><<<dim3(NG, 1), kNT1, Smem<N>::fwd(), s>>>(L, G, vbits, qlist, qcount, nullptr, nullptr, A,
                                                                nullptr, nullptr);
-    k_xline_herm<N, kLT><<<dim3(NH * TILES, 1), 16 * kLT, Smem<N>::xline(), s>>>(G, A, Rh, Gsp);
+    k_xline_fold<N><<<xline_grid<N>(1), XPlan<N>::NT, Smem<N>::xline(), s>>>(G, A, Rh, Gsp);
     const int T = t == 1 ? 1 : (t <= 4 ? 4 : 16);
     for (int out0 = 0; out0 < t; out0 += T) {
         const int nsel = t - out0 < T ? t - out0 : T;

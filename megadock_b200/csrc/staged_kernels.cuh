@@ -10,7 +10,7 @@
 //                    for the NG data rows y;
 //   K1c k_cols_fwd   (x-plane p, block of CB columns kz): pruned forward y-FFT
 //                    of the columns, in place in A -> A[p][ky][kz];
-//   K2  k_xline_herm (unchanged): x-FFT, conj(R^) product, Hermitian fold,
+//   K2  k_xline_fold (unchanged): x-FFT, conj(R^) product, Hermitian fold,
 //                    inverse x-FFT -> Gh[x][ky < N/2][kz];
 //   K3r k_rows_inv   (x, block of RB rows ky): inverse z-FFT in place in Gh;
 //   K3c k_cols_c2r   (x, block of CB columns z): unpack the half spectrum,
