@@ -80,9 +80,10 @@ int md_set_batch(md_ctx *ctx, int rotations_per_launch);
  * ligand and settings stay); the next docking call allocates them again for
  * its launch shape.  The autotuner calls it after trying large launch groups. */
 int md_release_work(md_ctx *ctx);
-/* Radix plan of the plane top-t (inverse plane) kernel: 0 the line plans,
- * 1 the kz split reversed, 2 the ky split reversed (t <= 4; larger t uses 0).
- * The autotuner (megadock_b200.tune) picks it together with the batch. */
+/* Radix plan of the inverse plane kernel (0, 1 or 2; other values are
+ * refused).  At FFT edge 128 it picks the line plans, the kz split reversed or
+ * the ky split reversed, and the autotuner (megadock_b200.tune) tries them;
+ * every other edge has one measured plan, and the call changes nothing. */
 int md_set_plan(md_ctx *ctx, int plan);
 /* Tile width asked of the x-line kernel (8, 16 or 32 kz lines; other values
  * are refused).  Every FFT size now runs the one tile shape that measured

@@ -18,17 +18,15 @@
 
 #include "../../include/md_b200.h"
 #include "dock_kernels.cuh"
+#include "inverse_kernels.cuh"
 #include "staged_kernels.cuh"
 
 using namespace mdb;
 
 namespace mdb {
 
-// Candidate groups per rotation from the top-t kernels: one per x-plane, or
-// one per (x-plane, column block) for the staged sizes.
-inline size_t cand_groups(size_t N) {
-    return N > (size_t)kMaxResidentN ? N * ((N + kCB - 1) / kCB) : N;
-}
+// Bound on the candidate groups per rotation of edge N (inv_groups).
+inline size_t cand_groups(size_t N) { return N * kMaxCluster; }
 
 // Per-launch intermediates for `cap` rotations of one launch group.
 struct WorkSet {
@@ -152,12 +150,10 @@ namespace mdb {
 template <int N>
 struct Sized {
     static constexpr int NG = N / 2;
-    static constexpr int NH = N / 2;
     static constexpr int TILES = (N + kLT - 1) / kLT;
     // above 224 the plane transforms run as row and column launches
     // (staged_kernels.cuh)
     static constexpr bool kStaged = staged<N>();
-    static constexpr int ZB = c2r_zblocks<N>();
     static size_t smem_fwd() { return (size_t)N * (N + 1) * sizeof(float2); }
     static size_t smem_xrec() { return (size_t)N * kLT * sizeof(float2); }
     static size_t smem_vox() { return vox_bits_smem<NG>(); }
@@ -182,8 +178,6 @@ struct Sized {
         else
             k_plane_fwd<N, MODE><<<dim3(NG, nb), kNT1, smem_fwd(), s>>>(L, G, vbits, qlist, qcount, sr, si, A, vr, vi);
     }
-    template <int V = 0>
-    static size_t smem_c2r() { return c2r_smem<N, V>(); }
 
     static cudaError_t set_attrs() {
         static bool done = false;
@@ -197,22 +191,12 @@ struct Sized {
             set((const void *)k_rows_fwd<N, 1>, rows_smem(N));
             set((const void *)k_rows_fwd<N, 2>, rows_smem(N));
             set((const void *)k_cols_fwd<N>, cols_fwd_smem(N));
-            set((const void *)k_rows_inv<N>, rows_smem(N));
-            set((const void *)k_cols_c2r<N, 1>, cols_c2r_smem(N));
-            set((const void *)k_cols_c2r<N, 4>, cols_c2r_smem(N));
-            set((const void *)k_cols_c2r<N, 16>, cols_c2r_smem(N));
         } else {
             set_fwd<0>(set);
             set_fwd<1>(set);
             set_fwd<2>(set);
-            set((const void *)k_plane_c2r<N, 1, 0>, smem_c2r<0>());
-            set((const void *)k_plane_c2r<N, 4, 0>, smem_c2r<0>());
-            set((const void *)k_plane_c2r<N, 16, 0>, smem_c2r<0>());
-            set((const void *)k_plane_c2r<N, 1, 1>, smem_c2r<1>());
-            set((const void *)k_plane_c2r<N, 4, 1>, smem_c2r<1>());
-            set((const void *)k_plane_c2r<N, 1, 2>, smem_c2r<2>());
-            set((const void *)k_plane_c2r<N, 4, 2>, smem_c2r<2>());
         }
+        if (e == cudaSuccess) e = set_inv_attrs<N>();
         set((const void *)k_xline_rec<N>, smem_xrec());
         set((const void *)k_vox_bits<NG, true>, smem_vox());
         set((const void *)k_vox_bits<NG, false>, smem_vox());
@@ -273,43 +257,6 @@ struct Sized {
         any_fwd<2>(c->stream, 1, L, G, w.vbits, w.qlist, w.qcount, nullptr, nullptr, nullptr, d_vr, d_vi);
     }
 
-    // The plane top-t kernel in passes of T candidates (T = 1, 4 or 16), with
-    // radix plan variant `plan` (T = 16 always uses variant 0).
-    template <int T, int V>
-    static void c2r(cudaStream_t s, const GridView &G, const float2 *Gh, int nb, int t, float nf3f, int out0,
-                    int nsel, Cand *cand) {
-        k_plane_c2r<N, T, V><<<dim3(N, nb), kNT, smem_c2r<V>(), s>>>(G, Gh, t, nf3f, out0, nsel, cand);
-    }
-    static void plane_topt(cudaStream_t s, const GridView &G, float2 *Gh, int nb, int t, float nf3f, Cand *cand,
-                           int plan) {
-        const int T = t == 1 ? 1 : (t <= 4 ? 4 : 16);
-        if constexpr (kStaged) {
-            k_rows_inv<N><<<dim3(N, (NH + kRB - 1) / kRB, nb), kNTS, rows_smem(N), s>>>(G, Gh);
-            for (int out0 = 0; out0 < t; out0 += T) {
-                const int nsel = std::min(T, t - out0);
-                const dim3 grid(N, ZB, nb);
-                if (T == 1) k_cols_c2r<N, 1><<<grid, kNTS, cols_c2r_smem(N), s>>>(G, Gh, t, out0, nsel, cand);
-                else if (T == 4) k_cols_c2r<N, 4><<<grid, kNTS, cols_c2r_smem(N), s>>>(G, Gh, t, out0, nsel, cand);
-                else k_cols_c2r<N, 16><<<grid, kNTS, cols_c2r_smem(N), s>>>(G, Gh, t, out0, nsel, cand);
-            }
-        } else {
-            for (int out0 = 0; out0 < t; out0 += T) {
-                const int nsel = std::min(T, t - out0);
-                if (T == 1) {
-                    if (plan == 1) c2r<1, 1>(s, G, Gh, nb, t, nf3f, out0, nsel, cand);
-                    else if (plan == 2) c2r<1, 2>(s, G, Gh, nb, t, nf3f, out0, nsel, cand);
-                    else c2r<1, 0>(s, G, Gh, nb, t, nf3f, out0, nsel, cand);
-                } else if (T == 4) {
-                    if (plan == 1) c2r<4, 1>(s, G, Gh, nb, t, nf3f, out0, nsel, cand);
-                    else if (plan == 2) c2r<4, 2>(s, G, Gh, nb, t, nf3f, out0, nsel, cand);
-                    else c2r<4, 0>(s, G, Gh, nb, t, nf3f, out0, nsel, cand);
-                } else {
-                    c2r<16, 0>(s, G, Gh, nb, t, nf3f, out0, nsel, cand);
-                }
-            }
-        }
-    }
-
     // One launch group: nb rotations whose matrices start at d_rot9, on work
     // set w and stream s.  With `ev` set, an event is recorded after each of
     // the five stages.
@@ -324,9 +271,9 @@ struct Sized {
         if (ev) cudaEventRecord(ev[2], s);
         k_xline_fold<N><<<xline_grid<N>(nb), XPlan<N>::NT, xline_smem<N>(), s>>>(G, w.A, c->d_Rh, w.G);
         if (ev) cudaEventRecord(ev[3], s);
-        plane_topt(s, G, w.G, nb, t, nf3f, w.cand, c->plan);
+        launch_inv<N>(s, G, w.G, nb, t, c->plan, w.cand);
         if (ev) cudaEventRecord(ev[4], s);
-        k_merge<<<nb, 256, 0, s>>>(w.cand, kStaged ? N * ZB : N, t, N, nf3f, rot0, d_pose);
+        k_merge<<<nb, 256, 0, s>>>(w.cand, inv_groups<N>(), t, N, nf3f, rot0, d_pose);
         if (ev) cudaEventRecord(ev[5], s);
     }
 };

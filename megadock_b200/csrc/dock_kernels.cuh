@@ -1188,74 +1188,187 @@ __device__ __forceinline__ Cand block_best(Cand mine, Cand *red) {
     return r;
 }
 
-// Per-thread sorted list of the T best (key, index) pairs seen, best first.
-// Empty slots hold (-inf, INT_MAX), which every non-NaN key beats, so the
-// one test against the last slot rejects NaN, too-small keys and equal keys
-// of later cells alike; an accepted key enters through a branch-free
-// compare-and-select network (the list is sorted, so "beats slot j" implies
-// "beats slot j+1").  Only candidates strictly after `floor` in selection
-// order are kept (used when a plane's top-t is found in several passes of T).
-template <int T>
-struct TopList {
-    float k[T];
-    int i[T];
-    __device__ __forceinline__ void init() {
+// The nsel best cells of a CTA's scores (nsel <= kSelMax), in selection order,
+// to out[0 .. nsel) (index -1 past the last).  item(it, o) computes the
+// scores of item it < COUNT -- o[k2].x of cell c0 + STEP k2 and o[k2].y of
+// cell c0 + STEP k2 + N -- and returns c0, or -1 when the item holds no cells
+// (never, with ALL).
+// With a floor (index >= 0) only cells after it in selection order compete.
+//
+// Every thread keeps the largest of its scores; each such maximum is the key
+// of a cell of its own, so the nsel-th largest of them bounds the nsel-th best
+// key from below.  Up to kSelLoose poses the bound is the largest over the
+// warps of each warp's nsel-th largest lane maximum (one barrier less); a peak
+// of the score spreads over the lanes of several warps, so for longer lists
+// that bound lets hundreds of cells through and the warps' sorted maxima are
+// merged instead.  The few threads that hold a score at or above the bound
+// recompute their items (the same bits) and append those cells to a shared
+// list; a cell's rank in the list (equal keys by the lower index) is its place
+// in the output.  A list longer than kSelCap (many equal keys) is found round
+// by round instead, every round rescanning the items for the best cell after
+// the last one.
+constexpr int kSelMax = 32;
+constexpr int kSelLoose = 3;
+constexpr int kSelCap = 256;
+template <int N, int NT, int COUNT, int Q2, int STEP, bool ALL, class Item>
+__device__ __forceinline__ void select_cells(const Item &item, int nsel, const Cand &floor, Cand *__restrict__ out) {
+    static_assert(NT % 32 == 0 && NT <= 1024, "whole warps");
+    constexpr int NW = NT / 32;
+    __shared__ float thr_w[NW];
+    __shared__ float thr_all;
+    // the warps' largest lane maxima, then the cells at or above the bound
+    __shared__ union {
+        float wtop[NW][kSelMax];
+        Cand list[kSelCap];
+    } sh;
+    __shared__ int nlist;
+    __shared__ Cand red[33];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int TRIPS = (COUNT + NT - 1) / NT;
+    const bool fl = floor.idx >= 0;
+    if (tid == 0) nlist = 0;
+    float tmax = -INFINITY;   // fmaxf drops NaN keys, which are never selected
+    if (!fl) {
 #pragma unroll
-        for (int j = 0; j < T; ++j) {
-            k[j] = -INFINITY;
-            i[j] = INT_MAX;
+        for (int r = 0; r < TRIPS; ++r) {
+            const int it = tid + r * NT;
+            if (COUNT % NT == 0 || it < COUNT) {
+                float2 o[Q2];
+                const int c0 = item(it, o);
+                float m = -INFINITY;
+                static_for<0, Q2>([&](auto k2_) {
+                    constexpr int k2 = decltype(k2_)::value;
+                    m = fmaxf(m, fmaxf(o[k2].x, o[k2].y));
+                });
+                // no branch: the trips' loads overlap
+                tmax = fmaxf(tmax, ALL || c0 >= 0 ? m : -INFINITY);
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int it = tid; it < COUNT; it += NT) {
+            float2 o[Q2];
+            const int c0 = item(it, o);
+            if (c0 < 0) continue;
+            static_for<0, Q2>([&](auto k2_) {
+                constexpr int k2 = decltype(k2_)::value;
+                if (key_better(floor.key, floor.idx, o[k2].x, c0 + STEP * k2)) tmax = fmaxf(tmax, o[k2].x);
+                if (key_better(floor.key, floor.idx, o[k2].y, c0 + STEP * k2 + N)) tmax = fmaxf(tmax, o[k2].y);
+            });
         }
     }
-    // FLOOR: a floor from an earlier pass is in force (uniform per launch).
-    template <bool FLOOR = true>
-    __device__ __forceinline__ void insert(float key, int idx, const Cand &floor) {
-        if (!((key > k[T - 1]) | ((key == k[T - 1]) & (idx < i[T - 1])))) return;
-        if (FLOOR && floor.idx >= 0 && !key_better(floor.key, floor.idx, key, idx)) return;
-        bool b[T];
-#pragma unroll
-        for (int j = 0; j < T; ++j) b[j] = (key > k[j]) | ((key == k[j]) & (idx < i[j]));
-#pragma unroll
-        for (int j = T - 1; j >= 1; --j) {
-            k[j] = b[j - 1] ? k[j - 1] : (b[j] ? key : k[j]);
-            i[j] = b[j - 1] ? i[j - 1] : (b[j] ? idx : i[j]);
+    {
+        float v = tmax, thw = -INFINITY;
+        for (int r = 0; r < nsel; ++r) {
+            const int vo = key_ord(v);
+            const int mo = __reduce_max_sync(0xffffffffu, vo);
+            thw = ord_key(mo);
+            if (nsel > kSelLoose && lane == 0) sh.wtop[warp][r] = thw;
+            const unsigned holders = __ballot_sync(0xffffffffu, vo == mo);
+            if (lane == __ffs(holders) - 1) v = -INFINITY;
         }
-        k[0] = b[0] ? key : k[0];
-        i[0] = b[0] ? idx : i[0];
+        if (lane == 0) thr_w[warp] = thw;
     }
-    // the best entry as a candidate (index -1 when the list is empty)
-    __device__ __forceinline__ Cand head() const { return Cand{k[0], i[0] == INT_MAX ? -1 : i[0]}; }
-    __device__ __forceinline__ void pop() {
+    __syncthreads();
+    float thr;
+    if (nsel <= kSelLoose) {
+        thr = thr_w[0];
 #pragma unroll
-        for (int j = 0; j < T - 1; ++j) {
-            k[j] = k[j + 1];
-            i[j] = i[j + 1];
+        for (int w = 1; w < NW; ++w) thr = fmaxf(thr, thr_w[w]);
+    } else {
+        if (warp == 0) {
+            int pos = 0;   // this lane's place in its warp's list
+            float best = -INFINITY;
+            for (int r = 0; r < nsel; ++r) {
+                const int vo = lane < NW && pos < nsel ? key_ord(sh.wtop[lane][pos]) : INT_MIN;
+                const int mo = __reduce_max_sync(0xffffffffu, vo);
+                best = ord_key(mo);
+                const unsigned holders = __ballot_sync(0xffffffffu, vo == mo);
+                if (lane == __ffs(holders) - 1) ++pos;
+            }
+            if (lane == 0) thr_all = best;
         }
-        k[T - 1] = -INFINITY;
-        i[T - 1] = INT_MAX;
+        __syncthreads();
+        thr = thr_all;
     }
-};
+    if (tmax >= thr) {
+#pragma unroll 1
+        for (int it = tid; it < COUNT; it += NT) {
+            float2 o[Q2];
+            const int c0 = item(it, o);
+            if (c0 < 0) continue;
+            auto enter = [&](float key, int idx) {
+                if (key >= thr && (!fl || key_better(floor.key, floor.idx, key, idx))) {
+                    const int e = atomicAdd(&nlist, 1);
+                    if (e < kSelCap) sh.list[e] = Cand{key, idx};
+                }
+            };
+            static_for<0, Q2>([&](auto k2_) {
+                constexpr int k2 = decltype(k2_)::value;
+                enter(o[k2].x, c0 + STEP * k2);
+                enter(o[k2].y, c0 + STEP * k2 + N);
+            });
+        }
+    }
+    __syncthreads();
+    const int n = nlist;
+    if (n <= kSelCap) {
+        for (int e = tid; e < n; e += NT) {
+            const Cand c = sh.list[e];
+            int rank = 0;
+            for (int f = 0; f < n; ++f) rank += key_better(sh.list[f].key, sh.list[f].idx, c.key, c.idx) ? 1 : 0;
+            if (rank < nsel) out[rank] = c;
+        }
+        if (tid >= n && tid < nsel) out[tid] = Cand{0.f, -1};
+        return;
+    }
+    Cand prev = floor;
+    for (int r = 0; r < nsel; ++r) {
+        Cand mine{0.f, -1};
+#pragma unroll 1
+        for (int it = tid; it < COUNT; it += NT) {
+            float2 o[Q2];
+            const int c0 = item(it, o);
+            if (c0 < 0) continue;
+            auto look = [&](float key, int idx) {
+                if (key != key || (prev.idx >= 0 && !key_better(prev.key, prev.idx, key, idx))) return;
+                if (mine.idx < 0 || key_better(key, idx, mine.key, mine.idx)) mine = Cand{key, idx};
+            };
+            static_for<0, Q2>([&](auto k2_) {
+                constexpr int k2 = decltype(k2_)::value;
+                look(o[k2].x, c0 + STEP * k2);
+                look(o[k2].y, c0 + STEP * k2 + N);
+            });
+        }
+        prev = block_best(mine, red);
+        if (tid == 0) out[r] = prev.idx >= 0 ? prev : Cand{0.f, -1};
+        if (prev.idx < 0) {
+            for (int r2 = r + 1 + tid; r2 < nsel; r2 += NT) out[r2] = Cand{0.f, -1};
+            break;
+        }
+    }
+}
 
 // K3: one x-plane of one rotation.  Input Gh[x][ky < N/2][kz] from
 // k_xline_fold.  (1) inverse FFT along kz of the N/2 rows, straight from
 // global memory; row 0 then holds h0 + i h_{N/2}, both real.  (2) complex-to-
 // real inverse along ky for every z column: with X the half spectrum,
 //   Z[k] = (X[k] + conj X[N/2-k]) + i w^k (X[k] - conj X[N/2-k]),  w = e^{2 pi i/N},
-// the N/2-point inverse FFT of Z gives s[2m] + i s[2m+1].  The scores feed a
-// per-thread top-T list directly (no score store), then a block merge writes
-// this plane's candidates cand[(b*N + x)*t + out0 + j] for j < nsel.
+// the N/2-point inverse FFT of Z gives s[2m] + i s[2m+1].  The plane's best
+// cells (select_cells) go to cand[(b*N + x)*t + out0 + j], j < nsel.
 // Keys are raw scores: ordering by raw equals ordering by raw / nf3 (a
 // positive constant), so the merge kernel divides only the winners.
-// Radix plans of this kernel, chosen per context by the autotuner: variant 0
-// uses the line plans of N (kz) and N/2 (ky), variant 1 reverses the kz split
-// (R2 x R1), variant 2 the ky split.  Three CTAs per SM (<= 42 registers)
-// where the radices are small enough.
+// Radix plans of this kernel, chosen per context by the autotuner: variant 1
+// reverses the kz split, any other is the line plans of N (kz) and N/2 (ky;
+// its two factors are equal).  Three CTAs per SM (<= 42 registers) where the
+// first kz radix is 8.
 constexpr int kC2RPlans = 3;
 template <int N, int V>
 struct C2RPlan {
     static constexpr int R1 = V == 1 ? Plan<N>::R2 : Plan<N>::R1;
     static constexpr int R2 = V == 1 ? Plan<N>::R1 : Plan<N>::R2;
-    static constexpr int Q1 = V == 2 ? Plan<N / 2>::R2 : Plan<N / 2>::R1;
-    static constexpr int Q2 = V == 2 ? Plan<N / 2>::R1 : Plan<N / 2>::R2;
+    static constexpr int Q1 = Plan<N / 2>::R1;
+    static constexpr int Q2 = Plan<N / 2>::R2;
 };
 
 // Shared memory of k_plane_c2r: the N/2 x PITCH plane.
@@ -1264,20 +1377,9 @@ constexpr size_t c2r_smem() {
     constexpr size_t PA = N + C2RPlan<N, V>::R1, PB = N + 8;
     return (size_t)(N / 2) * (PA > PB ? PA : PB) * sizeof(float2);
 }
-
-// Whether the plane kernel folds the half spectrum inside pass 1 of its ky
-// transform (both splits of the ky axis even).
-template <int N, int V>
-constexpr bool c2r_fold_ok() {
-    return N == 128 && C2RPlan<N, V>::Q1 % 2 == 0 && C2RPlan<N, V>::Q2 % 2 == 0;
-}
-
-template <int N, int T, int V = 0>
+template <int N, int V = 0>
 constexpr int c2r_min_blocks() {
-    using P = C2RPlan<N, V>;
-    constexpr size_t pitch = (size_t)N + (P::R1 > 8 ? P::R1 : 8);
-    if ((size_t)(N / 2) * pitch * 8 > 113 * 1024) return 1;   // one CTA per SM by shared memory
-    return (T <= 4 && P::R1 <= 8 && P::R2 <= 16 && P::Q1 <= 8 && P::Q2 <= 16) ? 3 : 2;
+    return C2RPlan<N, V>::R1 <= 8 ? 3 : 2;
 }
 
 // The plane kernel's item loops: items tid, tid + kNT, ... below COUNT, with
@@ -1288,11 +1390,10 @@ constexpr int c2r_min_blocks() {
     _Pragma("unroll") for (int r_##it = 0; r_##it < ((COUNT) + kNT - 1) / kNT; ++r_##it)       \
         if (const int it = tid + r_##it * kNT; ((COUNT) % kNT == 0) || it < (COUNT))
 
-template <int N, int T, int V = 0>
-__global__ void __launch_bounds__(kNT, c2r_min_blocks<N, T, V>())
-    k_plane_c2r(GridView G, const float2 *__restrict__ Gh, int t, float nf3f, int out0, int nsel,
-                Cand *__restrict__ cand) {
-    constexpr int NH = N / 2;
+template <int N, int V = 0>
+__global__ void __launch_bounds__(kNT, c2r_min_blocks<N, V>())
+    k_plane_c2r(GridView G, const float2 *__restrict__ Gh, int t, int out0, int nsel, Cand *__restrict__ cand) {
+    constexpr int NH = N / 2, NT = kNT;
     constexpr int R1 = C2RPlan<N, V>::R1, R2 = C2RPlan<N, V>::R2;
     constexpr int Q1 = C2RPlan<N, V>::Q1, Q2 = C2RPlan<N, V>::Q2;
     constexpr int PA = N + N / R2;   // step-1 layout: one pad per R2 block
@@ -1306,11 +1407,10 @@ __global__ void __launch_bounds__(kNT, c2r_min_blocks<N, T, V>())
     const int tid = threadIdx.x;
     const float2 *Gp = Gh + ((size_t)b * N + x) * NH * N;
 
-    // The z pass works on whole rows.  Where the rows split evenly over the
-    // warps (WZ), warp w owns rows [w NH/16, (w+1) NH/16) in both of its
-    // passes, so the passes are separated by warp barriers only; the plane
-    // barrier comes once, before the ky pass reads across rows.
-    constexpr bool WZ = kNT == 512 && NH % 16 == 0 && (NH / 16 * R2) % 32 == 0 && (NH / 16 * R1) % 32 == 0;
+    // The z pass works on whole rows: warp w owns rows [w NH/16, (w+1) NH/16) in
+    // both of its passes, so the passes are separated by warp barriers only; the
+    // plane barrier comes once, before the ky pass reads across rows.
+    static_assert(kNT == 512 && NH % 16 == 0 && (NH / 16 * R2) % 32 == 0 && (NH / 16 * R1) % 32 == 0, "warp rows");
     // (1a) inverse kz pass 1, straight from global: item = (row, t), t fastest
     auto z_pass1 = [&](int it) {
         const int row = it / R2, t = it % R2;
@@ -1327,46 +1427,37 @@ __global__ void __launch_bounds__(kNT, c2r_min_blocks<N, T, V>())
             S[row * PITCH + k1 * (R2 + 1) + t] = xv;
         });
     };
-    if constexpr (WZ) {
+    {
         constexpr int IPW = NH / 16 * R2;
 #pragma unroll
         for (int r = 0; r < IPW / 32; ++r) z_pass1((tid >> 5) * IPW + (tid & 31) + 32 * r);
         __syncwarp();
-    } else {
-        MDB_K3_ITEMS(it, NH * R2) { z_pass1(it); }
-        __syncthreads();
     }
-    // (1b) inverse kz pass 2: item = (row, u), u fastest; natural order after a barrier
+    // (1b) inverse kz pass 2: item = (row, u), u fastest; natural order after a warp barrier
     {
-        constexpr int IPW = WZ ? NH / 16 * R1 : 0;
-        constexpr int IPT = WZ ? IPW / 32 : (NH * R1 + kNT - 1) / kNT;
-        auto item = [&](int r) { return WZ ? (tid >> 5) * IPW + (tid & 31) + 32 * r : tid + r * kNT; };
+        constexpr int IPW = NH / 16 * R1, IPT = IPW / 32;
         float2 reg[IPT][R2];
 #pragma unroll
         for (int r = 0; r < IPT; ++r) {
-            const int it = item(r);
-            if (WZ || it < NH * R1) {
-                const int row = it / R1, u = it % R1;
-                static_for<0, R2>([&](auto n2_) {
-                    constexpr int n2 = decltype(n2_)::value;
-                    reg[r][n2] = S[row * PITCH + u * (R2 + 1) + n2];
-                });
-                Dft<R2, +1>::run(reg[r]);
-            }
+            const int it = (tid >> 5) * IPW + (tid & 31) + 32 * r;
+            const int row = it / R1, u = it % R1;
+            static_for<0, R2>([&](auto n2_) {
+                constexpr int n2 = decltype(n2_)::value;
+                reg[r][n2] = S[row * PITCH + u * (R2 + 1) + n2];
+            });
+            Dft<R2, +1>::run(reg[r]);
         }
-        if constexpr (WZ) __syncwarp();
-        else __syncthreads();
+        __syncwarp();
 #pragma unroll
         for (int r = 0; r < IPT; ++r) {
-            const int it = item(r);
-            if (WZ || it < NH * R1) {
-                const int row = it / R1, u = it % R1;
-                static_for<0, R2>([&](auto k2) { S[row * PITCH + u + R1 * k2] = reg[r][k2]; });
-            }
+            const int it = (tid >> 5) * IPW + (tid & 31) + 32 * r;
+            const int row = it / R1, u = it % R1;
+            static_for<0, R2>([&](auto k2) { S[row * PITCH + u + R1 * k2] = reg[r][k2]; });
         }
     }
+    static_assert(Q1 % 2 == 0 && Q2 % 2 == 0, "paired row sets");
     __syncthreads();
-    if constexpr (c2r_fold_ok<N, V>()) {
+    {
         // (2a + 2b) the fold into Z and pass 1 of the N/2-point inverse along
         // ky in one item.  Pass 1 item tt reads and writes the rows
         // tt + Q2 m; the fold partner N/2 - k of row k = tt + Q2 m is row
@@ -1457,186 +1548,27 @@ __global__ void __launch_bounds__(kNT, c2r_min_blocks<N, T, V>())
                 asm volatile("" ::: "memory");
             });
         }
-    } else {
-        // (2a) fold the half spectrum into Z, in place (pairs k, N/2-k)
-        MDB_K3_ITEMS(it, N * (NH / 2 + 1)) {
-            const int z = it % N, k = it / N;
-            if (k == 0) {
-                const float2 v = S[z];   // X0 + i X_{N/2}, both real
-                S[z] = make_float2(v.x + v.y, v.x - v.y);
-            } else {
-                const int k2 = NH - k;
-                const float2 a = S[k * PITCH + z], c = S[k2 * PITCH + z];
-                const float2 wk = conjf2(tw_at(k)), wk2 = conjf2(tw_at(k2));
-                // E = a + conj(c), D = a - conj(c), Z = E + i w^k D
-                const float2 e1 = make_float2(a.x + c.x, a.y - c.y), d1 = make_float2(a.x - c.x, a.y + c.y);
-                const float2 o1 = cmul(wk, d1);
-                const float2 z1 = make_float2(e1.x - o1.y, e1.y + o1.x);
-                if (k2 != k) {
-                    const float2 e2 = make_float2(c.x + a.x, c.y - a.y), d2 = make_float2(c.x - a.x, c.y + a.y);
-                    const float2 o2 = cmul(wk2, d2);
-                    S[k2 * PITCH + z] = make_float2(e2.x - o2.y, e2.y + o2.x);
-                }
-                S[k * PITCH + z] = z1;
-            }
-        }
-        __syncthreads();
-        // (2b) N/2-point inverse along ky, pass 1 (lanes = z), in place
-        MDB_K3_ITEMS(it, N * Q2) {
-            const int z = it % N, tt = it / N;
-            float2 v[Q1];
-            static_for<0, Q1>([&](auto m_) {
-                constexpr int mm = decltype(m_)::value;
-                v[mm] = S[(tt + Q2 * mm) * PITCH + z];
-            });
-            Dft<Q1, +1>::run(v);
-            static_for<0, Q1>([&](auto k1_) {
-                constexpr int k1 = decltype(k1_)::value;
-                float2 xv = v[k1];
-                if constexpr (k1 != 0) xv = cmul(xv, conjf2(tw_at(2 * tt * k1)));
-                S[(k1 * Q2 + tt) * PITCH + z] = xv;
-            });
-        }
     }
     __syncthreads();
-    // (2c) pass 2 -> scores s[2m], s[2m+1] -> per-thread top-T
-    TopList<T> top;
-    top.init();
-    Cand floor{0.f, -1};
+    // (2c) pass 2 -> scores s[2m], s[2m+1] -> the plane's best cells
     Cand *out = cand + ((size_t)b * N + x) * t + out0;
-    if (out0 > 0) {
-        floor = out[-1];
-        if (floor.idx < 0) {   // an earlier pass already ran out of cells
-            if (tid == 0)
-                for (int r = 0; r < nsel; ++r) out[r] = Cand{0.f, -1};
-            return;
-        }
+    const Cand floor = out0 > 0 ? out[-1] : Cand{0.f, -1};
+    if (out0 > 0 && floor.idx < 0) {   // an earlier pass already ran out of cells
+        if (tid < nsel) out[tid] = Cand{0.f, -1};
+        return;
     }
     const int base = x * N * N;
-    auto scan = [&](auto floor_on) {
-        constexpr bool FL = decltype(floor_on)::value;
-        for (int it = tid; it < N * Q1; it += blockDim.x) {
+    select_cells<N, NT, N * Q1, Q2, 2 * Q1 * N, true>(
+        [&](int it, float2(&o)[Q2]) {
             const int z = it % N, u = it / N;
-            float2 o[Q2];
             static_for<0, Q2>([&](auto n2_) {
                 constexpr int n2 = decltype(n2_)::value;
                 o[n2] = S[(u * Q2 + n2) * PITCH + z];
             });
             Dft<Q2, +1>::run(o);
-            const int cell0 = base + 2 * u * N + z;
-            static_for<0, Q2>([&](auto k2_) {
-                constexpr int k2 = decltype(k2_)::value;
-                constexpr int step = 2 * Q1 * k2 * N;   // 2 m2 N - 2 u N for m2 = u + Q1 k2
-                top.template insert<FL>(o[k2].x, cell0 + step, floor);
-                top.template insert<FL>(o[k2].y, cell0 + step + N, floor);
-            });
-        }
-    };
-    if (out0 > 0) {
-        // a later pass of T (t > T): the floor from the earlier passes is in
-        // force (out0 > 0 with no floor returned above)
-        scan(std::true_type{});
-    } else {
-        // (2c) pass 2: every item keeps only its thread's largest score; the
-        // pass's inputs stay in shared memory, so the few threads that pass
-        // the bound below recompute their items (the same bits) instead of
-        // every thread storing its scores (B200, N = 128: K3 193.4 -> 187.5 ms
-        // per 54,000 rotations, identical records).
-        float tmax = -INFINITY;   // fmaxf drops NaN keys, which are never selected
-        MDB_K3_ITEMS(it, N * Q1) {
-            const int z = it % N, u = it / N;
-            float2 o[Q2];
-            static_for<0, Q2>([&](auto n2_) {
-                constexpr int n2 = decltype(n2_)::value;
-                o[n2] = S[(u * Q2 + n2) * PITCH + z];
-            });
-            Dft<Q2, +1>::run(o);
-            static_for<0, Q2>([&](auto k2_) {
-                constexpr int k2 = decltype(k2_)::value;
-                tmax = fmaxf(tmax, fmaxf(o[k2].x, o[k2].y));
-            });
-        }
-        // Threshold: in each warp the nsel-th largest of its lanes' maxima is
-        // the key of nsel distinct cells of this plane, so the plane's nsel-th
-        // best key is at least that value; the largest such value over the
-        // warps bounds it too.  A cell below the bound cannot be among the
-        // plane's nsel best, so only cells at or above it enter the lists
-        // (equal keys still compete on the index inside the lists).
-        __shared__ float thr_w[kNT / 32];
-        {
-            const int lane = tid & 31, warp = tid >> 5;
-            float v = tmax, thw = -INFINITY;
-            for (int r = 0; r < nsel; ++r) {
-                const int vo = key_ord(v);
-                const int mo = __reduce_max_sync(0xffffffffu, vo);
-                if (mo == INT_MIN) {   // every lane NaN: no bound from this warp
-                    thw = NAN;
-                    break;
-                }
-                thw = ord_key(mo);
-                const unsigned holders = __ballot_sync(0xffffffffu, vo == mo);
-                if (lane == __ffs(holders) - 1) v = -INFINITY;
-            }
-            if (lane == 0) thr_w[warp] = thw;
-        }
-        __syncthreads();
-        float thr = thr_w[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) thr = fmaxf(thr, thr_w[w]);
-        // the few threads holding a score at or above the bound recompute
-        // their items and insert those scores
-        if (tmax >= thr) {
-            MDB_K3_ITEMS(it, N * Q1) {
-                const int z = it % N, u = it / N;
-                const int cell0 = base + 2 * u * N + z;
-                float2 o[Q2];
-                static_for<0, Q2>([&](auto n2_) {
-                    constexpr int n2 = decltype(n2_)::value;
-                    o[n2] = S[(u * Q2 + n2) * PITCH + z];
-                });
-                Dft<Q2, +1>::run(o);
-                static_for<0, Q2>([&](auto k2_) {
-                    constexpr int k2 = decltype(k2_)::value;
-                    constexpr int step = 2 * Q1 * k2 * N;
-                    const float2 s = o[k2];
-                    if (s.x >= thr) top.template insert<false>(s.x, cell0 + step, floor);
-                    if (s.y >= thr) top.template insert<false>(s.y, cell0 + step + N, floor);
-                });
-            }
-        }
-    }
-    // merge: each warp takes its best nsel from its lanes' lists (warp
-    // reductions only), then warp 0 takes the plane's best nsel from the
-    // warps' lists, with one block barrier in between
-    __shared__ Cand wl[kNT / 32][16];
-    const int lane = tid & 31, warp = tid >> 5;
-    if (__any_sync(0xffffffffu, top.i[0] != INT_MAX)) {
-        for (int r = 0; r < nsel; ++r) {
-            int owner;
-            const Cand c = warp_best(top.head(), owner);
-            if (lane == 0) wl[warp][r] = c;
-            if (c.idx >= 0 && lane == owner) top.pop();
-        }
-    } else if (lane < nsel) {
-        // no lane of this warp holds a candidate (the common case below the
-        // plane's threshold): its list is empty
-        wl[warp][lane] = Cand{0.f, -1};
-    }
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = blockDim.x >> 5;
-        int pos = 0;   // this lane's read position in its warp list
-        for (int r = 0; r < nsel; ++r) {
-            int owner;
-            const Cand c = warp_best((lane < nw && pos < nsel) ? wl[lane][pos] : Cand{0.f, -1}, owner);
-            if (lane == 0) out[r] = c.idx >= 0 ? c : Cand{0.f, -1};
-            if (c.idx < 0) {
-                if (lane == 0)
-                    for (int r2 = r + 1; r2 < nsel; ++r2) out[r2] = Cand{0.f, -1};
-                break;
-            }
-            if (lane == owner) ++pos;
-        }
-    }
+            return base + 2 * u * N + z;
+        },
+        nsel, floor, out);
 }
 
 // ------------------------------------------------------------------ K4

@@ -614,9 +614,8 @@ int md_dock_profile(md_ctx *ctx, const float *d_rot, int first_rot, int n_rot, i
     double acc[5] = {0, 0, 0, 0, 0};
     int nl = 0;
     // atom prep, marks, voxelizer, forward planes, x lines, one top-t pass per
-    // T poses, merge
-    const int T = t == 1 ? 1 : (t <= 4 ? 4 : 16);
-    const int per_group = 6 + (t + T - 1) / T;
+    // kSelMax poses, merge
+    const int per_group = 6 + (t + kSelMax - 1) / kSelMax;
     for (int r = 0; r < n_rot; r += B) {
         const int nb = std::min(B, n_rot - r);
         MD_CUDA(cudaEventRecord(ev[0], ctx->stream));

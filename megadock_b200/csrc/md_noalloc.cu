@@ -33,7 +33,7 @@
 #include <vector>
 
 #include "../../include/md_b200.h"
-#include "dock_kernels.cuh"
+#include "inverse_kernels.cuh"
 
 using namespace mdb;
 
@@ -42,6 +42,7 @@ namespace {
 constexpr size_t kScratchBytes = size_t(32) << 20;
 constexpr int kMaxN = 128;
 constexpr int kMaxT = 64;
+constexpr int kMaxNoallocCluster = 2;   // CTAs per plane of the inverse plans up to kMaxN
 constexpr int kMaxDevices = 64;
 // every grid-table size N <= kMaxN
 #define MDB_NOALLOC_SIZES(X)                                                                                  \
@@ -79,7 +80,6 @@ template <int N>
 struct Smem {
     static size_t fwd() { return (size_t)N * (N + 1) * sizeof(float2); }
     static size_t xline() { return xline_smem<N>(); }
-    static size_t c2r() { return c2r_smem<N, 0>(); }
 };
 
 template <int N>
@@ -90,9 +90,7 @@ cudaError_t set_attrs() {
     };
     set((const void *)k_plane_fwd<N, 0>, Smem<N>::fwd());
     set((const void *)k_xline_fold<N>, Smem<N>::xline());
-    set((const void *)k_plane_c2r<N, 1>, Smem<N>::c2r());
-    set((const void *)k_plane_c2r<N, 4>, Smem<N>::c2r());
-    set((const void *)k_plane_c2r<N, 16>, Smem<N>::c2r());
+    if (e == cudaSuccess) e = set_inv_attrs<N>();
     return e;
 }
 
@@ -156,17 +154,9 @@ void run_rotation(cudaStream_t s, const LigandView &L, const GridView &G, const 
     k_plane_fwd<N, 0><<<dim3(NG, 1), kNT1, Smem<N>::fwd(), s>>>(L, G, vbits, qlist, qcount, nullptr, nullptr, A,
                                                                nullptr, nullptr);
     k_xline_fold<N><<<xline_grid<N>(1), XPlan<N>::NT, Smem<N>::xline(), s>>>(G, A, Rh, Gsp);
-    const int T = t == 1 ? 1 : (t <= 4 ? 4 : 16);
-    for (int out0 = 0; out0 < t; out0 += T) {
-        const int nsel = t - out0 < T ? t - out0 : T;
-        if (T == 1)
-            k_plane_c2r<N, 1><<<dim3(N, 1), kNT, Smem<N>::c2r(), s>>>(G, Gsp, t, nf3f, out0, nsel, cand);
-        else if (T == 4)
-            k_plane_c2r<N, 4><<<dim3(N, 1), kNT, Smem<N>::c2r(), s>>>(G, Gsp, t, nf3f, out0, nsel, cand);
-        else
-            k_plane_c2r<N, 16><<<dim3(N, 1), kNT, Smem<N>::c2r(), s>>>(G, Gsp, t, nf3f, out0, nsel, cand);
-    }
-    k_merge<<<1, 256, 0, s>>>(cand, N, t, N, nf3f, rot, pose);
+    static_assert(inv_groups<N>() <= N * kMaxNoallocCluster, "candidate scratch");
+    launch_inv<N>(s, G, Gsp, 1, t, 0, cand);
+    k_merge<<<1, 256, 0, s>>>(cand, inv_groups<N>(), t, N, nf3f, rot, pose);
 }
 
 }  // namespace
@@ -184,7 +174,7 @@ extern "C" int md_dock_noalloc(int nf1, float grid_width, const float *d_grid_co
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t b_atom = up(sizeof(float4) * na), b_rad = up(sizeof(float2) * na);
     const size_t b_A = up(sizeof(float2) * NG * N * N), b_G = up(sizeof(float2) * N * (N / 2) * N);
-    const size_t b_cand = up(sizeof(Cand) * N * t);
+    const size_t b_cand = up(sizeof(Cand) * N * kMaxNoallocCluster * t);
     const size_t b_bits = up(sizeof(uint32_t) * NG * 2 * NG * ((NG + 31) / 32));
     const size_t b_ql = up(sizeof(int2) * NG * NG * NG), b_qc = up(sizeof(int) * NG);
     const size_t b_sr = up(sizeof(MarkEntry) * na), b_ss = up(sizeof(int) * (NG + 2 * kReach + 1));
