@@ -234,7 +234,8 @@ struct Sized {
     static void voxelize(md_ctx *c, const WorkSet &w, const float *d_rot9, int nb, cudaStream_t s) {
         GridView G{c->ng, c->gw, (float)(c->ng * c->gw) / 2, c->d_gc, c->d_tw};
         LigandView L{c->na, c->d_atom, c->d_rad2, c->delta};
-        k_atom_prep<NG><<<nb, kNTP, 0, s>>>(L, G, d_rot9, w.srec, w.sstart, w.cq, w.cstart);
+        const int nt = prep_threads(c->na);
+        k_atom_prep<NG><<<nb, nt, prep_smem<NG>(nt), s>>>(L, G, d_rot9, w.srec, w.sstart, w.cq, w.cstart);
         k_vox_mark<NG><<<dim3(NG, nb), kNT0, 0, s>>>(L, G, w.srec, w.sstart, w.marks);
         k_vox_bits<NG, true><<<dim3(NG, nb), kNT0, smem_vox(), s>>>(L, G, w.srec, w.sstart, w.cq, w.cstart,
                                                                    w.vbits, w.qlist, w.qcount, w.marks);

@@ -261,86 +261,126 @@ __device__ __forceinline__ int vox_code(const VoxShared<NG> &vs, int p, int q, i
 //  * charge entries cq[b][.] = (cell j * ng + k, charge bits) grouped by the
 //    charge cell's plane, in ascending atom order inside a bucket (the order
 //    in which MEGADOCK adds charges), bucket starts cstart[b][0 .. ng].
-constexpr int kNTP = 256;
+//
+// One CTA per rotation, its latency the whole cost of a small launch group.
+// The charge entries are a stable counting sort: warp w owns the w-th run of
+// atoms, counts its atoms per plane, and after one scan over (plane, warp)
+// writes them in atom order (one warp walking every atom before).  With the
+// charge sums from a shared list (k_vox_bits) instead of an array of NG^2 first
+// entries, the voxelizer stage went, in us per rotation (B200): N = 128, 1,544
+// atoms 0.67 -> 0.63; 160, 3,518 1.84 -> 1.48; 216, 10,074 8.8 -> 5.0; 256,
+// 12,000 15.0 -> 6.9; 330, 12,000 (8 rotations per launch) 53 -> 19.5.
+constexpr int kNTP = 256;            // threads for ligands of up to kPrepWide atoms
+constexpr int kNTPWide = 1024;       // threads above
+constexpr int kPrepWide = 3072;
+inline int prep_threads(int na) { return na <= kPrepWide ? kNTP : kNTPWide; }
+
+// Exclusive prefix sum of a[0 .. n) in place by the first warp; returns the total.
+__device__ __forceinline__ int warp_scan(int *a, int n) {
+    const int lane = threadIdx.x & 31;
+    int acc = 0;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+        const int i = i0 + lane;
+        const int v = i < n ? a[i] : 0;
+        int s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += u;
+        }
+        if (i < n) a[i] = acc + s - v;
+        acc += __shfl_sync(0xffffffffu, s, 31);
+    }
+    return acc;
+}
 
 template <int NG>
-__global__ void __launch_bounds__(kNTP)
+constexpr size_t prep_smem(int threads) {
+    return sizeof(int) * (size_t)(threads / 32) * NG;
+}
+
+template <int NG>
+__global__ void __launch_bounds__(kNTPWide)
     k_atom_prep(LigandView L, GridView G, const float *__restrict__ rotm, MarkEntry *__restrict__ rec,
                 int *__restrict__ sstart, int2 *__restrict__ cq, int *__restrict__ cstart) {
     constexpr int NBS = NG + 2 * kReach;
-    __shared__ int cnt_s[NBS], cnt_c[NG], cur_s[NBS], cur_c[NG];
+    extern __shared__ __align__(16) int wc[];   // [plane][warp] charge counts, then write positions
+    __shared__ int cnt_s[NBS], cnt_c[NG];
     __shared__ float m[9];
-    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     if (tid < 9) m[tid] = rotm[(size_t)b * 9 + tid];
     for (int i = tid; i < NBS; i += blockDim.x) cnt_s[i] = 0;
-    for (int i = tid; i < NG; i += blockDim.x) cnt_c[i] = 0;
+    for (int i = tid; i < NG * nw; i += blockDim.x) wc[i] = 0;
     __syncthreads();
-    for (int l = tid; l < L.na; l += blockDim.x) {
+    const int run = ((L.na + nw - 1) / nw + 31) & ~31;   // atoms per warp, whole steps of 32
+    const int l0 = min(warp * run, L.na), l1 = min(l0 + run, L.na);
+    for (int l = l0 + lane; l < l1; l += 32) {
         const float4 a = __ldg(&L.atom[l]);
         const float xr = rot_x(m, a.x, a.y, a.z);
         const int sb = box_origin(xr, G.gw, G.ng) + kReach;
         if (sb >= 0 && sb < NBS) atomicAdd(&cnt_s[sb], 1);
-        atomicAdd(&cnt_c[charge_cell(xr, G.pad, G.gw, G.ng)], 1);
+        atomicAdd(&wc[charge_cell(xr, G.pad, G.gw, G.ng) * nw + warp], 1);
     }
     __syncthreads();
     int *ss = sstart + (size_t)b * (NBS + 1);
     int *cs = cstart + (size_t)b * (NG + 1);
-    if (tid == 0) {
-        int acc = 0;
-        for (int i = 0; i < NBS; ++i) {
-            ss[i] = acc;
-            cur_s[i] = acc;
-            acc += cnt_s[i];
+    // plane totals, their starts, and each warp's start inside its planes
+    for (int i = tid; i < NG; i += blockDim.x) {
+        int n = 0;
+        for (int w = 0; w < nw; ++w) n += wc[i * nw + w];
+        cnt_c[i] = n;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const int n = warp_scan(cnt_s, NBS);
+        if (lane == 0) ss[NBS] = n;
+        const int nc = warp_scan(cnt_c, NG);
+        if (lane == 0) cs[NG] = nc;
+    }
+    __syncthreads();
+    for (int i = tid; i < NBS; i += blockDim.x) ss[i] = cnt_s[i];
+    for (int i = tid; i < NG; i += blockDim.x) {
+        int at = cnt_c[i];
+        cs[i] = at;
+        for (int w = 0; w < nw; ++w) {
+            const int n = wc[i * nw + w];
+            wc[i * nw + w] = at;
+            at += n;
         }
-        ss[NBS] = acc;
-        acc = 0;
-        for (int i = 0; i < NG; ++i) {
-            cs[i] = acc;
-            cur_c[i] = acc;
-            acc += cnt_c[i];
-        }
-        cs[NG] = acc;
     }
     __syncthreads();
     MarkEntry *rb = rec + (size_t)b * L.na;
-    for (int l = tid; l < L.na; l += blockDim.x) {
-        const float4 a = __ldg(&L.atom[l]);
-        const float xr = rot_x(m, a.x, a.y, a.z);
-        const int i2 = box_origin(xr, G.gw, G.ng);
-        const int sb = i2 + kReach;
-        if (sb < 0 || sb >= NBS) continue;
-        const float yr = rot_x(m + 3, a.x, a.y, a.z);
-        const float zr = rot_x(m + 6, a.x, a.y, a.z);
-        const float2 r2 = __ldg(&L.rad2[l]);
-        const int pos = atomicAdd(&cur_s[sb], 1);
-        rb[pos].pos = make_float4(xr, yr, zr, r2.x);
-        rb[pos].box = make_int4(i2, box_origin(yr, G.gw, G.ng), box_origin(zr, G.gw, G.ng), __float_as_int(r2.y));
-    }
-    // charge entries in atom order: warp 0 walks the atoms 32 at a time
-    if (tid < 32) {
-        int2 *qb = cq + (size_t)b * L.na;
-        for (int base = 0; base < L.na; base += 32) {
-            const int l = base + lane;
-            int ie = -1, key = 0;
-            float q = 0.f;
-            if (l < L.na) {
-                const float4 a = __ldg(&L.atom[l]);
-                ie = charge_cell(rot_x(m, a.x, a.y, a.z), G.pad, G.gw, G.ng);
-                const int je = charge_cell(rot_x(m + 3, a.x, a.y, a.z), G.pad, G.gw, G.ng);
-                const int ke = charge_cell(rot_x(m + 6, a.x, a.y, a.z), G.pad, G.gw, G.ng);
-                key = je * G.ng + ke;
-                q = a.w;
+    int2 *qb = cq + (size_t)b * L.na;
+    for (int base = l0; base < l1; base += 32) {
+        const int l = base + lane;
+        int ie = -1, key = 0;
+        float q = 0.f;
+        if (l < l1) {
+            const float4 a = __ldg(&L.atom[l]);
+            const float xr = rot_x(m, a.x, a.y, a.z);
+            const float yr = rot_x(m + 3, a.x, a.y, a.z);
+            const float zr = rot_x(m + 6, a.x, a.y, a.z);
+            const int i2 = box_origin(xr, G.gw, G.ng);
+            const int sb = i2 + kReach;
+            if (sb >= 0 && sb < NBS) {
+                const float2 r2 = __ldg(&L.rad2[l]);
+                const int pos = atomicAdd(&cnt_s[sb], 1);
+                rb[pos].pos = make_float4(xr, yr, zr, r2.x);
+                rb[pos].box = make_int4(i2, box_origin(yr, G.gw, G.ng), box_origin(zr, G.gw, G.ng), __float_as_int(r2.y));
             }
-            const uint32_t grp = __match_any_sync(0xffffffffu, ie);
-            int pos = 0;
-            if (ie >= 0) pos = cur_c[ie] + __popc(grp & ((1u << lane) - 1u));
-            __syncwarp();
-            if (ie >= 0) {
-                qb[pos] = make_int2(key, __float_as_int(q));
-                if (lane == 31 - __clz(grp)) cur_c[ie] += __popc(grp);
-            }
-            __syncwarp();
+            ie = charge_cell(xr, G.pad, G.gw, G.ng);
+            key = charge_cell(yr, G.pad, G.gw, G.ng) * G.ng + charge_cell(zr, G.pad, G.gw, G.ng);
+            q = a.w;
         }
+        const uint32_t grp = __match_any_sync(0xffffffffu, ie);
+        int pos = 0;
+        if (ie >= 0) pos = wc[ie * nw + warp] + __popc(grp & ((1u << lane) - 1u));
+        __syncwarp();
+        if (ie >= 0) {
+            qb[pos] = make_int2(key, __float_as_int(q));
+            if (lane == 31 - __clz(grp)) wc[ie * nw + warp] += __popc(grp);
+        }
+        __syncwarp();
     }
 }
 
@@ -409,25 +449,16 @@ constexpr bool vox_bits_dyn() {
     return sizeof(VoxShared<NG>) + sizeof(uint32_t) * 2 * NG * VoxShared<NG>::W > 40 * 1024;
 }
 
-// Whether k_vox_bits keeps the first charge entry of each cell in shared
-// memory (an int per cell): where it fits beside the dynamic bit planes in a
-// CTA's 227 KB (ng1 <= 200).  Above, each entry finds out whether it is its
-// cell's first by scanning the plane's earlier entries (a plane holds the
-// charges of a few hundred atoms at most).
-template <int NG>
-constexpr bool vox_first_smem() {
-    return sizeof(int) * NG * NG +
-               (vox_bits_dyn<NG>() ? sizeof(VoxShared<NG>) + sizeof(uint32_t) * 2 * NG * VoxShared<NG>::W : 0) <=
-           226 * 1024;   // a KB left for the kernel's static shared memory
-}
-
-// Dynamic shared memory of k_vox_bits: the first charge entry of each cell
-// (vox_first_smem), then (vox_bits_dyn) the bit planes and the output words.
+// Dynamic shared memory of k_vox_bits: the bit planes and the output words
+// (vox_bits_dyn).
 template <int NG>
 constexpr size_t vox_bits_smem() {
-    return (vox_first_smem<NG>() ? sizeof(int) * NG * NG : 0) +
-           (vox_bits_dyn<NG>() ? sizeof(VoxShared<NG>) + sizeof(uint32_t) * 2 * NG * VoxShared<NG>::W : 0);
+    return vox_bits_dyn<NG>() ? sizeof(VoxShared<NG>) + sizeof(uint32_t) * 2 * NG * VoxShared<NG>::W : 0;
 }
+
+// Charge entries of a plane k_vox_bits stages in shared memory; planes with
+// more (a ligand flattened into one plane) are read from global memory.
+constexpr int kVoxQ = 512;
 
 // PREMARKED: the marks come from K0m (marks != nullptr) instead of vox_mark.
 template <int NG, bool PREMARKED = false>
@@ -438,12 +469,12 @@ __global__ void __launch_bounds__(kNT0)
     constexpr int W = VoxShared<NG>::W;
     constexpr int NBS = NG + 2 * kReach;
     __shared__ int count;
-    constexpr bool FIRST = vox_first_smem<NG>();
-    extern __shared__ __align__(16) int first[];   // NG * NG where FIRST (vox_bits_smem)
+    __shared__ int2 qs[kVoxQ];
     VoxShared<NG> *vsp;
     uint32_t(*ob)[NG * W];
     if constexpr (vox_bits_dyn<NG>()) {
-        vsp = reinterpret_cast<VoxShared<NG> *>(first + (FIRST ? NG * NG : 0));
+        extern __shared__ __align__(16) unsigned char vox_smem[];
+        vsp = reinterpret_cast<VoxShared<NG> *>(vox_smem);
         ob = reinterpret_cast<uint32_t(*)[NG * W]>(vsp + 1);
     } else {
         __shared__ VoxShared<NG> vs_static;
@@ -472,9 +503,10 @@ __global__ void __launch_bounds__(kNT0)
         for (int w = tid; w < 5 * NG * W; w += blockDim.x) (&vs.core[0][0])[w] = 0u;
         for (int w = tid; w < 3 * NG * W; w += blockDim.x) (&vs.surf[0][0])[w] = 0u;
     }
-    for (int w = tid; w < 2 * NG * W; w += blockDim.x) (&ob[0][0])[w] = 0u;
-    if constexpr (FIRST)
-        for (int c = tid; c < NG * NG; c += blockDim.x) first[c] = 0x7fffffff;
+    // this plane's charge entries, in atom order
+    const int c0 = cstart[(size_t)b * (NG + 1) + p], nq = cstart[(size_t)b * (NG + 1) + p + 1] - c0;
+    const int2 *qb = cq + (size_t)b * L.na + c0;
+    for (int e = tid; e < min(nq, kVoxQ); e += blockDim.x) qs[e] = qb[e];
     if (tid == 0) count = 0;
     __syncthreads();
     if constexpr (!PREMARKED) {
@@ -492,30 +524,30 @@ __global__ void __launch_bounds__(kNT0)
         ob[1][q * W + w] = c1 & valid;
     }
     // charges of this plane, in atom order: the first entry of each cell sums
-    // that cell's entries in order
-    const int c0 = cstart[(size_t)b * (NG + 1) + p], c1 = cstart[(size_t)b * (NG + 1) + p + 1];
-    const int2 *qb = cq + (size_t)b * L.na;
-    if constexpr (FIRST) {
-        for (int e = c0 + tid; e < c1; e += blockDim.x) atomicMin(&first[qb[e].x], e);
-        __syncthreads();
-    }
+    // that cell's entries in order.  Every thread walks the whole list, the
+    // same entry in all lanes at a time (a broadcast from shared memory; a
+    // plane holds the charges of some tens to hundreds of atoms).
     int2 *ql = qlist + ((size_t)b * NG + p) * NG * NG;
-    for (int e = c0 + tid; e < c1; e += blockDim.x) {
-        const int key = qb[e].x;
-        if constexpr (FIRST) {
-            if (first[key] != e) continue;
-        } else {
+    auto sum_cells = [&](const int2 *ent) {
+        for (int e = tid; e < nq; e += blockDim.x) {
+            const int key = ent[e].x;
             bool later = false;
-            for (int f = c0; f < e && !later; ++f) later = qb[f].x == key;
-            if (later) continue;
+            float acc = 0.f;
+            for (int f = 0; f < nq; ++f) {
+                const int2 v = ent[f];
+                if (v.x != key) continue;
+                if (f < e) {
+                    later = true;
+                    break;
+                }
+                acc = __fadd_rn(acc, __int_as_float(v.y));
+            }
+            if (!later) ql[atomicAdd(&count, 1)] = make_int2(key, __float_as_int(acc));
         }
-        float acc = 0.f;
-        for (int f = e; f < c1; ++f) {
-            const int2 v = qb[f];
-            if (v.x == key) acc = __fadd_rn(acc, __int_as_float(v.y));
-        }
-        ql[atomicAdd(&count, 1)] = make_int2(key, __float_as_int(acc));
-    }
+    };
+    if (nq <= kVoxQ) sum_cells(qs);
+    else sum_cells(qb);
+    __syncthreads();
     uint32_t *dst = vbits + ((size_t)b * NG + p) * 2 * NG * W;
     for (int w = tid; w < 2 * NG * W; w += blockDim.x) dst[w] = (&ob[0][0])[w];
     __syncthreads();
