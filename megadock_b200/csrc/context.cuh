@@ -187,9 +187,9 @@ struct Sized {
             if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         };
         if constexpr (kStaged) {
-            set((const void *)k_rows_fwd<N, 0>, rows_smem(N));
-            set((const void *)k_rows_fwd<N, 1>, rows_smem(N));
-            set((const void *)k_rows_fwd<N, 2>, rows_smem(N));
+            set((const void *)k_rows_fwd<N, 0>, rows_smem<N>());
+            set((const void *)k_rows_fwd<N, 1>, rows_smem<N>());
+            set((const void *)k_rows_fwd<N, 2>, rows_smem<N>());
             set((const void *)k_cols_fwd<N>, cols_fwd_smem(N));
         } else {
             set_fwd<0>(set);
@@ -211,7 +211,7 @@ struct Sized {
     static void staged_fwd(cudaStream_t s, int nb, const LigandView &L, const GridView &G, const uint32_t *vbits,
                            const int2 *qlist, const int *qcount, const float *sr, const float *si, float2 *A,
                            float *vr, float *vi) {
-        k_rows_fwd<N, MODE><<<dim3(NG, (NG + kRB - 1) / kRB, nb), kNTS, rows_smem(N), s>>>(L, G, vbits, qlist, qcount,
+        k_rows_fwd<N, MODE><<<dim3(NG, (NG + kRB - 1) / kRB, nb), kNTS, rows_smem<N>(), s>>>(L, G, vbits, qlist, qcount,
                                                                                            sr, si, A, vr, vi);
         if constexpr (MODE != 2) k_cols_fwd<N><<<dim3(NG, (N + kCB - 1) / kCB, nb), kNTS, cols_fwd_smem(N), s>>>(G, A);
     }
