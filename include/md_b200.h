@@ -74,7 +74,9 @@ int md_ligand_data(md_ctx *ctx, int na, const float *xyz_centred, const float *r
                    float lig_core);
 
 /* Rotations per launch for md_dock (1 = the plain per-rotation pipeline;
- * > 1 = the batched form, launched as one captured CUDA graph). */
+ * > 1 = the batched form, launched as one captured CUDA graph).  A context
+ * that never gets a value launches groups of rotations that fit a work set of
+ * 1 GiB (one rotation where even that has no room), without a graph. */
 int md_set_batch(md_ctx *ctx, int rotations_per_launch);
 /* Free the context's rotation work buffers and captured graphs (receptor,
  * ligand and settings stay); the next docking call allocates them again for

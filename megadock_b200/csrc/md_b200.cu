@@ -121,6 +121,23 @@ int carve_scratch(md_ctx *ctx, const size_t *sz, int n, char **out) {
     return MD_OK;
 }
 
+// Rotations per launch of a call over n: md_set_batch's value, or, in a context
+// that never got one, as many as keep the work set within kAutoBytes, at most
+// kAutoGroup, in groups of even size.  One rotation leaves most of the GPU
+// idle (64 to 2,000 CTAs a kernel at N = 128) and pays nine launches: B200,
+// 360 rotations at N = 128, t = 3, from host buffers: 30.5 -> 4.3 ms.
+constexpr size_t kAutoBytes = size_t(1) << 30;
+constexpr int kAutoGroup = 64;
+int group_of(const md_ctx *ctx, int n, int t) {
+    if (ctx->batch) return std::max(1, std::min(ctx->batch, n));
+    const WorkSet::Sizes z = WorkSet::need(1, ctx->N, t, std::max(ctx->na, 1));
+    size_t one = 0;
+    for (size_t b : z.b) one += b;
+    const int most = (int)std::max<size_t>(1, std::min<size_t>(kAutoGroup, kAutoBytes / one));
+    const int groups = (std::max(n, 1) + most - 1) / most;
+    return std::max(1, (n + groups - 1) / groups);
+}
+
 int check_ready(md_ctx *ctx) {
     if (!ctx->N) {
         ctx->err = "md_set_grid has not been called";
@@ -139,13 +156,22 @@ int check_ready(md_ctx *ctx) {
 
 // The rotation loop of one md_dock call on device buffers.
 int run_dock(md_ctx *ctx, const float *d_rot, int first_rot, int n_rot, int t, DevPose *d_pose) {
-    const int B = std::max(1, std::min(ctx->batch, n_rot));
-    int rc = ensure_work(ctx, B, t, B == 1 ? 1 : ctx->lanes);
+    int B = group_of(ctx, n_rot, t);
+    const bool batched = ctx->batch != 0 && B > 1;
+    int rc = ensure_work(ctx, B, t, batched ? ctx->lanes : 1);
+    if (rc && ctx->batch == 0 && B > 1) {
+        // no room for the automatic group: one rotation at a time
+        cudaGetLastError();
+        B = 1;
+        rc = ensure_work(ctx, B, t);
+    }
     if (rc) return rc;
-    if (B == 1) {
-        // plain form: one rotation per fused pipeline, launched back to back
-        for (int r = 0; r < n_rot; ++r)
-            launch_dock(ctx, 0, ctx->stream, d_rot + 9 * (size_t)r, 1, first_rot + r, t, d_pose + (size_t)r * t);
+    if (!batched) {
+        // plain form (one rotation per fused pipeline) and automatic groups,
+        // launched back to back
+        for (int r = 0; r < n_rot; r += B)
+            launch_dock(ctx, 0, ctx->stream, d_rot + 9 * (size_t)r, std::min(B, n_rot - r), first_rot + r, t,
+                        d_pose + (size_t)r * t);
         MD_CUDA(cudaGetLastError());
         return MD_OK;
     }
@@ -607,7 +633,7 @@ int md_dock_profile(md_ctx *ctx, const float *d_rot, int first_rot, int n_rot, i
     int rc = check_ready(ctx);
     if (rc) return rc;
     MD_CUDA(cudaSetDevice(ctx->device));
-    const int B = std::max(1, std::min(ctx->batch, n_rot));
+    const int B = group_of(ctx, n_rot, t);
     if ((rc = ensure_work(ctx, B, t))) return rc;
     cudaEvent_t ev[6];
     for (auto &e : ev) MD_CUDA(cudaEventCreate(&e));
@@ -657,7 +683,7 @@ int md_dock_pairs(md_ctx *runner, md_ctx *const *pairs, int npairs, const float 
             return rc;
         }
         MD_CUDA(set_attrs(c->N));
-        const int B = std::max(1, std::min(c->batch, std::max(n_rot[p], 1)));
+        const int B = group_of(c, n_rot[p], t);
         const WorkSet::Sizes zp = WorkSet::need(B, c->N, t, std::max(c->na, 1));
         for (int k = 0; k < WorkSet::kBufs; ++k) z.b[k] = std::max(z.b[k], zp.b[k]);
         // the pair's (uid, gen) stands for every argument the capture takes
@@ -682,7 +708,7 @@ int md_dock_pairs(md_ctx *runner, md_ctx *const *pairs, int npairs, const float 
         int group = 0;
         for (int p = 0; p < npairs; ++p) {
             md_ctx *c = pairs[p];
-            const int B = std::max(1, std::min(c->batch, std::max(n_rot[p], 1)));
+            const int B = group_of(c, n_rot[p], t);
             DevPose *out = reinterpret_cast<DevPose *>(d_out[p]);
             for (int r = 0; r < n_rot[p]; r += B, ++group) {
                 const int nb = std::min(B, n_rot[p] - r);
@@ -721,7 +747,7 @@ int adjoint_core(md_ctx *ctx, const float *rotmat, int n, const int4 *shift, con
     MD_CUDA(cudaSetDevice(ctx->device));
     const int N = ctx->N, ng = ctx->ng;
     const size_t ng3 = (size_t)ng * ng * ng;
-    const int B = std::max(1, std::min(ctx->batch, n));
+    const int B = group_of(ctx, n, 1);
     int rc = ensure_work(ctx, B, 1);
     if (rc) return rc;
     const size_t sz[8] = {sizeof(float) * 9 * n,       sizeof(float) * n,
@@ -900,7 +926,7 @@ int md_pose_scores(md_ctx *ctx, const float *rotmat, int n, const md_pose *poses
         }
         shift[r] = make_int4(poses[r].i, poses[r].j, poses[r].k, 0);
     }
-    const int B = std::max(1, std::min(ctx->batch, n));
+    const int B = group_of(ctx, n, 1);
     if ((rc = ensure_work(ctx, B, 1))) return rc;
     const size_t sz[4] = {sizeof(float) * 9 * n, sizeof(int4) * n, sizeof(float) * n, sizeof(float) * 2 * ng3 * B};
     char *p[4];
@@ -951,7 +977,7 @@ int md_pose_terms(md_ctx *ctx, const float *rec_rpsc, const float *rotmat, int n
     const size_t ng3 = (size_t)ng * ng * ng;
     // poses per launch: their voxel grids within about 1 GB
     const int P = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, ((size_t)1 << 30) / (8 * ng3)));
-    const int B = std::max(1, std::min(ctx->batch, P));
+    const int B = group_of(ctx, P, 1);
     if ((rc = ensure_work(ctx, B, 1))) return rc;
     float *d_rot = nullptr, *d_vox = nullptr, *d_terms = nullptr, *d_rpsc = nullptr;
     int4 *d_tem = nullptr;
