@@ -99,6 +99,7 @@ struct md_ctx {
     // grid
     int N = 0, ng = 0;
     float gw = 0.f;
+    float gc_step = 0.f;   // grid_coord[1] - grid_coord[0], the cell width the receptor field reads
     float *d_gc = nullptr;
     float2 *d_tw = nullptr;
     // receptor spectrum [kx][ky][kz] and the receptor voxel grids (for the adjoint)

@@ -308,6 +308,7 @@ int md_set_grid(md_ctx *ctx, int nf1, float grid_width, const float *grid_coord)
     }
     if (ctx->gw != grid_width) free_graphs(ctx);   // the grid width is a kernel argument
     ctx->gw = grid_width;
+    ctx->gc_step = grid_coord[1] - grid_coord[0];
     MD_CUDA(cudaMemcpyAsync(ctx->d_gc, grid_coord, sizeof(float) * ctx->ng, cudaMemcpyHostToDevice, ctx->stream));
     MD_CUDA(cudaStreamSynchronize(ctx->stream));
     return MD_OK;
@@ -356,127 +357,73 @@ int md_receptor_build(md_ctx *ctx, int na, const float *xyz_centred, const float
         if (rc) return rc;
     }
     const size_t ng3 = (size_t)ng * ng * ng;
-    const float open_space = -7777.0f;
-    // host copies of the two grid-coordinate values the reference reads
-    std::vector<float> gc(ng);
-    MD_CUDA(cudaMemcpy(gc.data(), ctx->d_gc, sizeof(float) * ng, cudaMemcpyDeviceToHost));
     RecParams P;
     P.ng = ng;
     P.na = na;
     P.gw = ctx->gw;
-    P.width = gc[1] - gc[0];
+    P.width = ctx->gc_step;
     P.eps_core = rec_core;
     P.e_ratio = elec_ratio;
     P.cpg = -1 * P.width * 80.0f / (-2800.0f * elec_ratio);
     P.ace_ratio = (double)ace_ratio;
     P.reach_core = (int)((2.4 + ctx->gw - 0.01) / ctx->gw);
     P.reach_shell = (int)((12 + ctx->gw - 0.01) / ctx->gw);
-    float *d_xyz = nullptr, *d_rad = nullptr, *d_q = nullptr, *d_ace = nullptr, *d_grid = nullptr;
-    RecAtom *d_atoms = nullptr;
-    int *d_cnt = nullptr, *d_start = nullptr, *d_list = nullptr;
-    void *d_masks = nullptr;   // sweep row masks above ng = kRecSmemNg
+    const int words = (ng + 63) / 64;
+    const size_t mask = sizeof(unsigned long long) * words * ng * ng;
+    const size_t sz[6] = {sizeof(float) * 6 * na, sizeof(RecAtom) * na, mask, mask, mask,
+                          make_receptor ? 0 : sizeof(float) * 2 * ng3};
+    char *p[6];
+    int rc = carve_scratch(ctx, sz, 6, p);
+    if (rc) return rc;
+    const float *d_in = reinterpret_cast<float *>(p[0]);
+    RecAtom *d_atoms = reinterpret_cast<RecAtom *>(p[1]);
+    float *d_r = make_receptor ? ctx->d_recv : reinterpret_cast<float *>(p[5]);
+    float *d_i = d_r + ng3;
+    cudaStream_t s = ctx->stream;
+    // one upload: coordinates, radii, charges, ACE values
+    std::vector<float> in(6 * (size_t)na);
+    std::copy(xyz_centred, xyz_centred + 3 * (size_t)na, in.begin());
+    std::copy(radius, radius + na, in.begin() + 3 * (size_t)na);
+    std::copy(charge, charge + na, in.begin() + 4 * (size_t)na);
+    std::copy(ace, ace + na, in.begin() + 5 * (size_t)na);
     cudaError_t e = cudaSuccess;
     auto step = [&](cudaError_t x) {
         if (e == cudaSuccess) e = x;
     };
-    auto cleanup = [&]() {
-        cudaFree(d_xyz);
-        cudaFree(d_rad);
-        cudaFree(d_q);
-        cudaFree(d_ace);
-        cudaFree(d_atoms);
-        cudaFree(d_cnt);
-        cudaFree(d_start);
-        cudaFree(d_list);
-        cudaFree(d_masks);
-        if (!make_receptor) cudaFree(d_grid);
-    };
-    cudaStream_t s = ctx->stream;
-    step(cudaMalloc(&d_xyz, sizeof(float) * 3 * na));
-    step(cudaMalloc(&d_rad, sizeof(float) * na));
-    step(cudaMalloc(&d_q, sizeof(float) * na));
-    step(cudaMalloc(&d_ace, sizeof(float) * na));
-    step(cudaMalloc(&d_atoms, sizeof(RecAtom) * na));
-    step(cudaMalloc(&d_cnt, sizeof(int) * (ng * ng + 1)));
-    step(cudaMalloc(&d_start, sizeof(int) * (ng * ng + 1)));
-    if (make_receptor) d_grid = ctx->d_recv;
-    else step(cudaMalloc(&d_grid, sizeof(float) * 2 * ng3));
-    if (e != cudaSuccess) {
-        cleanup();
-        ctx->err = std::string("receptor grids: ") + cudaGetErrorString(e);
-        return MD_ERR_CUDA;
-    }
-    float *d_r = d_grid, *d_i = d_grid + ng3;
-    step(cudaMemcpyAsync(d_xyz, xyz_centred, sizeof(float) * 3 * na, cudaMemcpyHostToDevice, s));
-    step(cudaMemcpyAsync(d_rad, radius, sizeof(float) * na, cudaMemcpyHostToDevice, s));
-    step(cudaMemcpyAsync(d_q, charge, sizeof(float) * na, cudaMemcpyHostToDevice, s));
-    step(cudaMemcpyAsync(d_ace, ace, sizeof(float) * na, cudaMemcpyHostToDevice, s));
-    step(cudaMemsetAsync(d_r, 0, sizeof(float) * ng3, s));
-    const int rows = ng * ng;
-    // the two propagation sweeps: row masks of ceil(ng / 64) words, in shared
-    // memory up to ng = kRecSmemNg, else in a global buffer
-    auto sweep = [&]() {
-        if (ng <= kRecSmemNg) {
-            const size_t smem = sizeof(RowMask<2>) * rows;
-            step(cudaFuncSetAttribute(k_rec_sweep<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(sizeof(RowMask<2>) * kRecSmemNg * kRecSmemNg)));
-            for (int k = 0; k < 2 && e == cudaSuccess; ++k)
-                k_rec_sweep<2, false><<<1, 1024, smem, s>>>(P, d_r, open_space, nullptr);
-        } else if (ng <= 192) {
-            step(cudaMalloc(&d_masks, sizeof(RowMask<3>) * rows));
-            for (int k = 0; k < 2 && e == cudaSuccess; ++k)
-                k_rec_sweep<3, true><<<1, 1024, 0, s>>>(P, d_r, open_space, static_cast<RowMask<3> *>(d_masks));
-        } else {
-            step(cudaMalloc(&d_masks, sizeof(RowMask<4>) * rows));
-            for (int k = 0; k < 2 && e == cudaSuccess; ++k)
-                k_rec_sweep<4, true><<<1, 1024, 0, s>>>(P, d_r, open_space, static_cast<RowMask<4> *>(d_masks));
+    step(cudaMemcpyAsync(p[0], in.data(), sizeof(float) * in.size(), cudaMemcpyHostToDevice, s));
+    // a core value of 0 makes every cell of the zeroed grid compare equal to
+    // the core, NaN none; equal to the open-space marker, core cells are open
+    step(cudaMemsetAsync(p[2], rec_core == 0.0f ? 0xff : 0, mask, s));
+    step(cudaMemsetAsync(p[3], 0, mask, s));
+    const bool draw_core = rec_core != 0.0f && !std::isnan(rec_core);
+    const int core_open = rec_core == kRecOpen;
+    auto build = [&](auto words_, auto km_) {
+        constexpr int W = decltype(words_)::value, KM = decltype(km_)::value;
+        RowMask<W> *core = reinterpret_cast<RowMask<W> *>(p[2]), *open = reinterpret_cast<RowMask<W> *>(p[3]),
+                   *reach = reinterpret_cast<RowMask<W> *>(p[4]);
+        k_rec_prep<<<(na + 255) / 256, 256, 0, s>>>(P, d_in, d_in + 3 * (size_t)na, d_in + 4 * (size_t)na,
+                                                    d_in + 5 * (size_t)na, d_atoms);
+        if (draw_core) k_rec_core<W><<<na, 32, 0, s>>>(P, d_atoms, ctx->d_gc, core);
+        k_rec_rays<W><<<dim3((ng * ng + 63) / 64, 3), 64, 0, s>>>(P, core, open, core_open);
+        for (int k = 0; k < 2; ++k) {
+            k_rec_sweep<W><<<1, (ng + 31) & ~31, 0, s>>>(P, core, open, reach);
+            k_rec_apply<W><<<(ng * ng + 127) / 128, 128, 0, s>>>(P, core, open, reach);
         }
-    };
-    const int cells_blocks = (int)((ng3 + 255) / 256);
-    std::vector<int> cnt(rows + 1), start(rows + 1);
-    auto scan = [&](int n) {   // counts -> starts on the host (n + 1 entries)
-        step(cudaMemcpyAsync(cnt.data(), d_cnt, sizeof(int) * n, cudaMemcpyDeviceToHost, s));
-        step(cudaStreamSynchronize(s));
-        start[0] = 0;
-        for (int r = 0; r < n; ++r) start[r + 1] = start[r] + cnt[r];
-        step(cudaMemcpyAsync(d_start, start.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s));
-        return start[n];
+        k_rec_cells<W, KM><<<dim3(ng, (ng + kRecRows - 1) / kRecRows), 32 * kRecRows, 0, s>>>(
+            P, d_atoms, ctx->d_gc, core, open, core_open, d_r, d_i);
     };
     if (e == cudaSuccess) {
-        k_rec_prep<<<(na + 255) / 256, 256, 0, s>>>(P, d_xyz, d_rad, d_q, d_ace, d_atoms);
-        k_rec_core<<<na, 128, 0, s>>>(P, d_atoms, ctx->d_gc, d_r);
-        k_rec_rays<<<(3 * rows + 255) / 256, 256, 0, s>>>(P, d_r, open_space);
-        sweep();
-        k_rec_final<<<cells_blocks, 256, 0, s>>>(P, d_r, open_space);
-        // surface shell over per-row atom lists
-        k_rec_rows<<<(rows + 3) / 4, 128, 0, s>>>(P, d_atoms, ctx->d_gc, d_cnt, nullptr, nullptr);
-        const int nlist = scan(rows);
-        step(cudaMalloc(&d_list, sizeof(int) * std::max(1, nlist)));
-        if (e == cudaSuccess) {
-            k_rec_rows<<<(rows + 3) / 4, 128, 0, s>>>(P, d_atoms, ctx->d_gc, d_cnt, d_start, d_list);
-            k_rec_shell<<<cells_blocks, 256, 0, s>>>(P, d_atoms, ctx->d_gc, d_start, d_list, d_r);
-            step(cudaGetLastError());
-            step(cudaStreamSynchronize(s));
-            cudaFree(d_list);
-            d_list = nullptr;
-        }
-        // electrostatics over per-plane charged-atom lists
-        if (e == cudaSuccess) {
-            k_rec_planes<<<(ng + 3) / 4, 128, 0, s>>>(P, d_atoms, d_cnt, nullptr, nullptr);
-            const int nplane = scan(ng);
-            step(cudaMalloc(&d_list, sizeof(int) * std::max(1, nplane)));
-        }
-        if (e == cudaSuccess) {
-            k_rec_planes<<<(ng + 3) / 4, 128, 0, s>>>(P, d_atoms, d_cnt, d_start, d_list);
-            k_rec_elec<<<cells_blocks, 256, 0, s>>>(P, d_atoms, ctx->d_gc, d_start, d_list, d_r, d_i);
-            if (make_receptor) launch_receptor(ctx, d_r, d_i);
-            step(cudaGetLastError());
-        }
+        if (ng <= 32) build(std::integral_constant<int, 1>{}, std::integral_constant<int, 1>{});
+        else if (ng <= 64) build(std::integral_constant<int, 1>{}, std::integral_constant<int, 2>{});
+        else if (ng <= 128) build(std::integral_constant<int, 2>{}, std::integral_constant<int, 4>{});
+        else if (ng <= 192) build(std::integral_constant<int, 3>{}, std::integral_constant<int, 6>{});
+        else build(std::integral_constant<int, 4>{}, std::integral_constant<int, 8>{});
+        if (make_receptor) launch_receptor(ctx, d_r, d_i);
+        step(cudaGetLastError());
         if (grid_r) step(cudaMemcpyAsync(grid_r, d_r, sizeof(float) * ng3, cudaMemcpyDeviceToHost, s));
         if (grid_i) step(cudaMemcpyAsync(grid_i, d_i, sizeof(float) * ng3, cudaMemcpyDeviceToHost, s));
-        step(cudaStreamSynchronize(s));
     }
-    cleanup();
+    step(cudaStreamSynchronize(s));
     if (e != cudaSuccess) {
         ctx->err = std::string("receptor grids: ") + cudaGetErrorString(e);
         return MD_ERR_CUDA;

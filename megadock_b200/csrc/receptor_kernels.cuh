@@ -2,18 +2,18 @@
 // (Receptor::rpscace, src/receptor.cpp:20-254; Receptor::electro, :258-346).
 //
 //   K_r0 k_rec_prep    per atom: centre cell, squared radii, ACE term, field reach
-//   K_r1 k_rec_core    per atom: core value in the cube of +-reach cells within 1.5 R^2
+//   K_r1 k_rec_core    per atom: core bits in the cube of +-reach cells within 1.5 R^2
 //   K_r2 k_rec_rays    per line and axis: open space reachable straight from a face
-//   K_r3 k_rec_sweep   two in-place 6-neighbour propagation sweeps (see below)
-//   K_r4 k_rec_final   cavities -> core, open space -> 0
-//   K_r5 k_rec_rows    per (i, j) row, the atoms whose shell reaches it, in atom order
-//   K_r6 k_rec_shell   per cell: sum over those atoms of 1 - 0.8 ACE (double, rounded per add)
-//   K_r7 k_rec_planes  per x plane, the charged atoms whose cube reaches it, in atom order
-//   K_r8 k_rec_elec    per non-core cell: sum over those atoms of e beta q / eps(r) / r
+//   K_r3 k_rec_sweep   in-place 6-neighbour propagation sweep (see below), twice,
+//   K_r4 k_rec_apply   each followed by the backward neighbours
+//   K_r5 k_rec_cells   per cell: shell sum of 1 - 0.8 ACE (double, rounded per add)
+//                      and field sum of e beta q / eps(r) / r over the atoms in order
 //
-// Every float operation is an explicitly rounded intrinsic in the reference's
-// association order, and every sum runs over atoms in ascending order, so the
-// grids equal the sequential CPU result.
+// Core, open space and the rest are bit masks, one row of cells along z per
+// RowMask, until the last kernel writes the two float grids.  Every float
+// operation is an explicitly rounded intrinsic in the reference's association
+// order, and every sum runs over atoms in ascending order, so the grids equal
+// the sequential CPU result.
 //
 // The propagation sweep visits cells in linear order c = (i, j, k) and, for an
 // open cell with 1 <= i <= ng-2 and 2 <= j, k <= ng-2 ("valid"), opens its zero
@@ -23,18 +23,15 @@
 //     R(c) = O(c) | (Z(c) & OR_p (V(p) & R(p)))
 // which depends only on rows (i, j-1) and (i-1, j) and on the row itself, so
 // rows on the same anti-diagonal i + j are independent: one CTA walks the
-// 2 ng - 1 anti-diagonals, a warp per row, R kept as bit masks in shared
-// memory.  Zero cells next to a valid open successor (k+1, j+1 or i+1) are
-// opened too, after their own visit, so they do not propagate in that sweep.
+// 2 ng - 1 anti-diagonals, a thread per row, the previous diagonal's masks in
+// shared memory and the next one's inputs already on their way.  Zero cells
+// next to a valid open successor (k+1, j+1 or i+1) are opened too, after their
+// own visit, so they do not propagate in that sweep.
 #pragma once
 #include <cstdint>
 
 namespace mdb {
 
-// Row masks of the propagation sweep: ceil(ng / 64) 64-bit words per (i, j)
-// row.  Up to ng = 112 every row's mask fits one CTA's shared memory (two
-// words, 16 B x 112^2); larger grids keep them in a global scratch buffer.
-constexpr int kRecSmemNg = 112;
 constexpr int kRecMaxNg = 256;
 
 struct RecAtom {
@@ -43,7 +40,7 @@ struct RecAtom {
     int iw, jw, kw;       // centre cell of the field, (int)(c / width + ng/2)
     float core2, shell2;  // 1.5 R^2 and (R + 3.6)^2
     double term;          // 1 + ACE (-0.8) ratio
-    float q;
+    float cq;             // e_ratio * -2800 * q
     int reach_e;          // field cube half width (-1: uncharged)
 };
 
@@ -53,6 +50,10 @@ struct RecParams {
     double ace_ratio;
     int reach_core, reach_shell;
 };
+
+// Value of the open-space marker of Receptor::rpscace; a core value (-d) equal
+// to it, to 0 or NaN changes what the comparisons with the core value mean.
+constexpr float kRecOpen = -7777.0f;
 
 __device__ __forceinline__ float rec_sq(float c, float g) {
     const float d = __fsub_rn(c, g);
@@ -81,7 +82,7 @@ __global__ void k_rec_prep(RecParams P, const float *__restrict__ xyz, const flo
     a.term = __dadd_rn(1.0, __dmul_rn(__dmul_rn((double)ace[l], -0.8), P.ace_ratio));
     const float q = charge[l];
     const float aq = fabsf(q);
-    a.q = q;
+    a.cq = __fmul_rn(__fmul_rn(P.e_ratio, -2800.0f), q);
     if (aq <= 1.0e-6f) a.reach_e = -1;
     else if ((double)aq < 0.07) a.reach_e = 4;
     else if ((double)aq < 0.21) a.reach_e = 5;
@@ -89,255 +90,316 @@ __global__ void k_rec_prep(RecParams P, const float *__restrict__ xyz, const flo
     A[l] = a;
 }
 
+// Bits of one row of cells along z, k in [0, ng).
+template <int WORDS>
+struct RowMask {
+    unsigned long long w[WORDS];
+};
+
+// bits lo <= k <= hi of word w
+__device__ __forceinline__ unsigned long long word_range(int w, int lo, int hi) {
+    lo = max(lo - 64 * w, 0);
+    hi = min(hi - 64 * w, 63);
+    if (hi < lo) return 0ull;
+    return ((hi - lo == 63) ? ~0ull : ((1ull << (hi - lo + 1)) - 1ull)) << lo;
+}
+
+template <int WORDS>
 __global__ void k_rec_core(RecParams P, const RecAtom *__restrict__ A, const float *__restrict__ gc,
-                           float *__restrict__ grid) {
+                           RowMask<WORDS> *__restrict__ core) {
     const int l = blockIdx.x;
     const RecAtom a = A[l];
     const int ng = P.ng, R = P.reach_core;
     const int i0 = max(a.io - R, 0), i1 = min(a.io + R + 1, ng);
     const int j0 = max(a.jo - R, 0), j1 = min(a.jo + R + 1, ng);
     const int k0 = max(a.ko - R, 0), k1 = min(a.ko + R + 1, ng);
-    const int ni = max(i1 - i0, 0), nj = max(j1 - j0, 0), nk = max(k1 - k0, 0);
-    for (int t = threadIdx.x; t < ni * nj * nk; t += blockDim.x) {
-        const int i = i0 + t / (nj * nk), j = j0 + (t / nk) % nj, k = k0 + t % nk;
-        const float d = __fadd_rn(__fadd_rn(rec_sq(a.x, gc[i]), rec_sq(a.y, gc[j])), rec_sq(a.z, gc[k]));
-        if (d < a.core2) grid[((size_t)i * ng + j) * ng + k] = P.eps_core;
+    const int ni = max(i1 - i0, 0), nj = max(j1 - j0, 0);
+    for (int t = threadIdx.x; t < ni * nj; t += blockDim.x) {
+        const int i = i0 + t / nj, j = j0 + t % nj;
+        const float dxy = __fadd_rn(rec_sq(a.x, gc[i]), rec_sq(a.y, gc[j]));
+        unsigned long long m = 0ull;
+        int w = k0 >> 6;
+        for (int k = k0; k < k1; ++k) {
+            if ((k >> 6) != w) {
+                if (m) atomicOr(&core[i * ng + j].w[w], m);
+                m = 0ull;
+                w = k >> 6;
+            }
+            if (__fadd_rn(dxy, rec_sq(a.z, gc[k])) < a.core2) m |= 1ull << (k & 63);
+        }
+        if (m) atomicOr(&core[i * ng + j].w[w], m);
     }
 }
 
-// one thread per (a, b, axis): walk in from both faces until a core cell
-__global__ void k_rec_rays(RecParams P, float *__restrict__ grid, float open_space) {
+// Open space seen straight from the six faces, ORed into open (zero at the
+// start): blockIdx.y = axis; a thread per word column along x and y, per row
+// along z.
+template <int WORDS>
+__global__ void k_rec_rays(RecParams P, const RowMask<WORDS> *__restrict__ core, RowMask<WORDS> *__restrict__ open,
+                           int core_open) {
     const int ng = P.ng;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 3 * ng * ng) return;
-    const int ax = t / (ng * ng), a = (t / ng) % ng, b = t % ng;
-    const size_t ng2 = (size_t)ng * ng;
-    size_t base, step;
-    if (ax == 0) {
-        base = (size_t)a + (size_t)ng * b;
-        step = ng2;
-    } else if (ax == 1) {
-        base = (size_t)b * ng2 + (size_t)a * ng;
-        step = 1;
-    } else {
-        base = (size_t)a * ng2 + b;
-        step = ng;
+    if (blockIdx.y == 2) {
+        if (t >= ng * ng) return;
+        const RowMask<WORDS> c = core[t];
+        int first = ng, last = -1;   // first and last core cell of the row
+#pragma unroll
+        for (int w = WORDS - 1; w >= 0; --w)
+            if (c.w[w]) first = 64 * w + __ffsll((long long)c.w[w]) - 1;
+#pragma unroll
+        for (int w = 0; w < WORDS; ++w)
+            if (c.w[w]) last = 64 * w + 63 - __clzll((long long)c.w[w]);
+#pragma unroll
+        for (int w = 0; w < WORDS; ++w) {
+            unsigned long long m = word_range(w, 0, first - 1) | word_range(w, last + 1, ng - 1);
+            if (core_open) m |= c.w[w];
+            if (m) atomicOr(&open[t].w[w], m);
+        }
+        return;
     }
+    if (t >= ng * WORDS) return;
+    const int a = t / WORDS, w = t % WORDS;
+    const size_t base = blockIdx.y == 0 ? (size_t)a : (size_t)a * ng, step = blockIdx.y == 0 ? ng : 1;
+    const unsigned long long valid = word_range(w, 0, ng - 1);
+    unsigned long long run = valid;
+#pragma unroll 8
     for (int k = 0; k < ng; ++k) {
-        float *v = &grid[base + step * k];
-        if (*v == P.eps_core) break;
-        *v = open_space;
+        run &= ~core[base + step * k].w[w];
+        if (run) atomicOr(&open[base + step * k].w[w], run);
     }
+    run = valid;
+#pragma unroll 8
     for (int k = ng - 1; k >= 0; --k) {
-        float *v = &grid[base + step * k];
-        if (*v == P.eps_core) break;
-        *v = open_space;
+        run &= ~core[base + step * k].w[w];
+        if (run) atomicOr(&open[base + step * k].w[w], run);
     }
 }
 
-template <int WORDS>
-struct RowMask {
-    unsigned long long w[WORDS];
-};
+__device__ __forceinline__ bool rec_vrow(int i, int j, int ng) { return i >= 1 && i <= ng - 2 && j >= 2 && j <= ng - 2; }
 
+// One propagation sweep: R of every row from the open cells and the zero cells
+// (neither core nor open).  One CTA, a thread per row of the anti-diagonal.
 template <int WORDS>
-__device__ __forceinline__ bool mbit(const RowMask<WORDS> &m, int k) {
-    return (m.w[k >> 6] >> (k & 63)) & 1ull;
-}
-
-// One propagation sweep; one CTA.  The R masks of every row (ng^2 of them)
-// live in dynamic shared memory, or with GMEM in `gmask` (ng^2 entries).
-template <int WORDS, bool GMEM>
-__global__ void __launch_bounds__(1024)
-    k_rec_sweep(RecParams P, float *__restrict__ grid, float open_space, RowMask<WORDS> *__restrict__ gmask) {
-    extern __shared__ __align__(16) unsigned char rec_smem[];
-    RowMask<WORDS> *Rm = GMEM ? gmask : reinterpret_cast<RowMask<WORDS> *>(rec_smem);
-    const int ng = P.ng;
-    const size_t ng2 = (size_t)ng * ng;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-    auto vrow = [&](int i, int j) { return i >= 1 && i <= ng - 2 && j >= 2 && j <= ng - 2; };
+__global__ void __launch_bounds__(kRecMaxNg)
+    k_rec_sweep(RecParams P, const RowMask<WORDS> *__restrict__ core, const RowMask<WORDS> *__restrict__ open,
+                RowMask<WORDS> *__restrict__ reach) {
+    __shared__ RowMask<WORDS> diag[2][kRecMaxNg];   // R of the last two anti-diagonals, by i
+    const int ng = P.ng, i = threadIdx.x;
+    RowMask<WORDS> Vk, all;   // positions 2 <= k <= ng - 2 (as a source on the k axis); 0 <= k < ng
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+        Vk.w[w] = word_range(w, 2, ng - 2);
+        all.w[w] = word_range(w, 0, ng - 1);
+    }
+    auto inside = [&](int d) { return i < ng && d - i >= 0 && d - i < ng; };
+    RowMask<WORDS> c{}, o{};
+    if (inside(0)) {
+        c = core[(size_t)i * ng - i];
+        o = open[(size_t)i * ng - i];
+    }
     for (int d = 0; d <= 2 * (ng - 1); ++d) {
-        const int ilo = max(0, d - (ng - 1)), ihi = min(ng - 1, d);
-        for (int i = ilo + warp; i <= ihi; i += nwarps) {
+        const RowMask<WORDS> C = c, O = o;
+        if (inside(d + 1)) {
+            c = core[(size_t)i * ng + (d + 1 - i)];
+            o = open[(size_t)i * ng + (d + 1 - i)];
+        }
+        if (inside(d)) {
             const int j = d - i;
-            const float *row = grid + (size_t)i * ng2 + (size_t)j * ng;
-            RowMask<WORDS> O{}, Z{};
-            for (int k0 = 0; k0 < ng; k0 += 32) {
-                const int k = k0 + lane;
-                const float v = k < ng ? row[k] : 1.0f;
-                const unsigned o = __ballot_sync(0xffffffffu, k < ng && v == open_space);
-                const unsigned z = __ballot_sync(0xffffffffu, k < ng && v == 0.0f);
-                O.w[k0 >> 6] |= (unsigned long long)o << (k0 & 63);
-                Z.w[k0 >> 6] |= (unsigned long long)z << (k0 & 63);
+            RowMask<WORDS> In{};
+            if (j > 0 && rec_vrow(i, j - 1, ng)) {
+#pragma unroll
+                for (int w = 0; w < WORDS; ++w) In.w[w] |= diag[(d + 1) & 1][i].w[w];
             }
-            if (lane == 0) {
-                RowMask<WORDS> In{};
-                if (j > 0 && vrow(i, j - 1)) {
-                    const RowMask<WORDS> q = Rm[(size_t)i * ng + j - 1];
+            if (i > 0 && rec_vrow(i - 1, j, ng)) {
 #pragma unroll
-                    for (int w = 0; w < WORDS; ++w) In.w[w] |= q.w[w];
-                }
-                if (i > 0 && vrow(i - 1, j)) {
-                    const RowMask<WORDS> q = Rm[(size_t)(i - 1) * ng + j];
-#pragma unroll
-                    for (int w = 0; w < WORDS; ++w) In.w[w] |= q.w[w];
-                }
-                const bool vr = vrow(i, j);
-                // Vk: positions 2 <= k <= ng - 2 (as a source on the k axis)
-                RowMask<WORDS> Vk{};
-#pragma unroll
-                for (int w = 0; w < WORDS; ++w) {
-                    const int lo = max(2 - 64 * w, 0), hi = min(ng - 2 - 64 * w, 63);   // bit range in word w
-                    if (hi >= lo)
-                        Vk.w[w] = ((hi - lo == 63) ? ~0ull : ((1ull << (hi - lo + 1)) - 1ull)) << lo;
-                }
-                // seeds S = O | (Z & In & Vk); k receives from k - 1 when
-                // P(k) = Z(k) & Vk(k - 1) & vr.  R = S | (P & (R << 1)) is a
-                // carry chain: within a run of P, everything from the first
-                // position after a reached cell up to the run's end is reached,
-                // i.e. P & (~(P + B) | B) with B = (R << 1) & P restricted to
-                // the seeds (the addition carries through the run); a run
-                // crossing a word boundary takes the previous word's top bit
-                // of R as its carry in.
-                RowMask<WORDS> R{};
-                unsigned long long carry = 0ull;   // R at bit 63 of the previous word
-#pragma unroll
-                for (int w = 0; w < WORDS; ++w) {
-                    const unsigned long long S = O.w[w] | (Z.w[w] & In.w[w] & Vk.w[w]);
-                    const unsigned long long vprev = (Vk.w[w] << 1) | (w ? (Vk.w[w - 1] >> 63) : 0ull);
-                    const unsigned long long P = vr ? (Z.w[w] & vprev) : 0ull;
-                    const unsigned long long B = ((S << 1) | carry) & P;
-                    const unsigned long long r = S | (P & (~(P + B) | B));
-                    R.w[w] = r;
-                    carry = r >> 63;
-                }
-                Rm[(size_t)i * ng + j] = R;
+                for (int w = 0; w < WORDS; ++w) In.w[w] |= diag[(d + 1) & 1][i - 1].w[w];
             }
-            __syncwarp();
+            const bool vr = rec_vrow(i, j, ng);
+            // seeds S = O | (Z & In & Vk); k receives from k - 1 when
+            // P(k) = Z(k) & Vk(k - 1) & vr.  R = S | (P & (R << 1)) is a
+            // carry chain: within a run of P, everything from the first
+            // position after a reached cell up to the run's end is reached,
+            // i.e. P & (~(P + B) | B) with B = (R << 1) & P restricted to
+            // the seeds (the addition carries through the run); a run
+            // crossing a word boundary takes the previous word's top bit
+            // of R as its carry in.
+            RowMask<WORDS> R{};
+            unsigned long long carry = 0ull;   // R at bit 63 of the previous word
+#pragma unroll
+            for (int w = 0; w < WORDS; ++w) {
+                const unsigned long long Z = all.w[w] & ~(C.w[w] | O.w[w]);
+                const unsigned long long S = O.w[w] | (Z & In.w[w] & Vk.w[w]);
+                const unsigned long long vprev = (Vk.w[w] << 1) | (w ? (Vk.w[w ? w - 1 : 0] >> 63) : 0ull);
+                const unsigned long long Pm = vr ? (Z & vprev) : 0ull;
+                const unsigned long long B = ((S << 1) | carry) & Pm;
+                const unsigned long long r = S | (Pm & (~(Pm + B) | B));
+                R.w[w] = r;
+                carry = r >> 63;
+            }
+            diag[d & 1][i] = R;
+            reach[(size_t)i * ng + j] = R;
         }
         __syncthreads();
     }
-    // apply: forward-reached cells, then zero cells with a valid reached successor
-    for (size_t c = threadIdx.x; c < ng2 * ng; c += blockDim.x) {
-        const int i = (int)(c / ng2), j = (int)((c / ng) % ng), k = (int)(c % ng);
-        const RowMask<WORDS> &r = Rm[(size_t)i * ng + j];
-        if (mbit(r, k)) continue;   // written below, after every read of this sweep
-        if (grid[c] != 0.0f) continue;
-        bool b = false;
-        if (k + 1 < ng && vrow(i, j) && k + 1 >= 2 && k + 1 <= ng - 2 && mbit(r, k + 1)) b = true;
-        if (!b && j + 1 < ng && vrow(i, j + 1) && k >= 2 && k <= ng - 2 && mbit(Rm[(size_t)i * ng + j + 1], k)) b = true;
-        if (!b && i + 1 < ng && vrow(i + 1, j) && k >= 2 && k <= ng - 2 && mbit(Rm[(size_t)(i + 1) * ng + j], k)) b = true;
-        if (b) grid[c] = open_space;
-    }
-    __syncthreads();
-    for (size_t c = threadIdx.x; c < ng2 * ng; c += blockDim.x) {
-        const int i = (int)(c / ng2), j = (int)((c / ng) % ng), k = (int)(c % ng);
-        if (mbit(Rm[(size_t)i * ng + j], k)) grid[c] = open_space;
-    }
 }
 
-__global__ void k_rec_final(RecParams P, float *__restrict__ grid, float open_space) {
-    const size_t ng3 = (size_t)P.ng * P.ng * P.ng;
-    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < ng3; c += (size_t)gridDim.x * blockDim.x) {
-        const float v = grid[c];
-        if (v == 0.0f) grid[c] = P.eps_core;
-        else if (v == open_space) grid[c] = 0.0f;
-    }
-}
-
-// Atoms (in order) whose shell cube and sphere reach row (i, j): one warp per
-// row, 32 atoms per step, compacted in order with a ballot.  count pass
-// (out == nullptr) writes cnt[row]; fill pass writes out[start[row] ..].
-__global__ void k_rec_rows(RecParams P, const RecAtom *__restrict__ A, const float *__restrict__ gc,
-                           int *__restrict__ cnt, const int *__restrict__ start, int *__restrict__ out) {
-    const int row = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
+// After a sweep: the reached cells are open, and so are zero cells with a
+// valid reached successor.
+template <int WORDS>
+__global__ void k_rec_apply(RecParams P, const RowMask<WORDS> *__restrict__ core, RowMask<WORDS> *__restrict__ open,
+                            const RowMask<WORDS> *__restrict__ reach) {
     const int ng = P.ng;
-    if (row >= ng * ng) return;   // whole warps
-    const int i = row / ng, j = row % ng;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= ng * ng) return;
+    const int i = t / ng, j = t % ng;
+    const RowMask<WORDS> R = reach[t], C = core[t], O = open[t];
+    RowMask<WORDS> back{};
+    if (rec_vrow(i, j, ng)) {
+#pragma unroll
+        for (int w = 0; w < WORDS; ++w) {
+            const unsigned long long lo = R.w[w] & word_range(w, 2, ng - 2);
+            const unsigned long long hi = w + 1 < WORDS ? R.w[w + 1 < WORDS ? w + 1 : w] & word_range(w + 1, 2, ng - 2) : 0ull;
+            back.w[w] = (lo >> 1) | (hi << 63);
+        }
+    }
+    if (j + 1 < ng && rec_vrow(i, j + 1, ng)) {
+#pragma unroll
+        for (int w = 0; w < WORDS; ++w) back.w[w] |= reach[t + 1].w[w] & word_range(w, 2, ng - 2);
+    }
+    if (i + 1 < ng && rec_vrow(i + 1, j, ng)) {
+#pragma unroll
+        for (int w = 0; w < WORDS; ++w) back.w[w] |= reach[t + ng].w[w] & word_range(w, 2, ng - 2);
+    }
+    RowMask<WORDS> out;
+#pragma unroll
+    for (int w = 0; w < WORDS; ++w) {
+        const unsigned long long Z = word_range(w, 0, ng - 1) & ~(C.w[w] | O.w[w]);
+        out.w[w] = O.w[w] | R.w[w] | (Z & back.w[w]);
+    }
+    open[t] = out;
+}
+
+// The two grids.  CTA = (i, kRecRows rows j), a warp per row, lane = k modulo
+// 32 with KM = ceil(ng / 32) cells each.  The atoms are walked once, in order:
+// the CTA collects those whose shell or field cube touches its rows into a
+// shared list (ballot compaction keeps the order), then every warp adds the
+// listed atoms' terms to its cells from registers.
+constexpr int kRecRows = 8;
+constexpr int kRecList = 512;
+
+struct RecEntry {
+    float x, y, z, shell2;   // shell2 < 0: the atom's shell cube misses this CTA
+    double term;
+    float cq, cq4, cq80;     // e_ratio -2800 q, over 4 and over 80 (the two constant dielectrics)
+    int jo, ko, jw, kw, reach_e;   // reach_e < 0: no field here
+};
+
+template <int WORDS, int KM>
+__global__ void __launch_bounds__(32 * kRecRows)
+    k_rec_cells(RecParams P, const RecAtom *__restrict__ A, const float *__restrict__ gc,
+                const RowMask<WORDS> *__restrict__ core, const RowMask<WORDS> *__restrict__ open, int core_open,
+                float *__restrict__ grid_r, float *__restrict__ grid_i) {
+    constexpr int NT = 32 * kRecRows;
+    __shared__ RecEntry list[kRecList];
+    __shared__ int wcount[kRecRows];
+    const int ng = P.ng, i = blockIdx.x, jb = blockIdx.y * kRecRows;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int j = jb + warp, je = min(jb + kRecRows, ng) - 1;
     const int R = P.reach_shell;
-    int n = 0;
-    const int base = out ? start[row] : 0;
-    for (int l0 = 0; l0 < P.na; l0 += 32) {
-        const int l = l0 + lane;
-        bool hit = false;
+    const float gi = gc[i], gj = gc[min(j, ng - 1)];
+    float gk[KM], shell[KM], field[KM];
+#pragma unroll
+    for (int m = 0; m < KM; ++m) {
+        gk[m] = gc[min(lane + 32 * m, ng - 1)];
+        shell[m] = 0.f;
+        field[m] = 0.f;
+    }
+    int n = 0;   // entries in the list (the same in every thread)
+    for (int l0 = 0; l0 < P.na; l0 += NT) {
+        const int l = l0 + tid;
+        bool hs = false, he = false;
+        RecAtom a;
         if (l < P.na) {
-            const RecAtom &a = A[l];
-            hit = !(i < a.io - R || i > a.io + R || j < a.jo - R || j > a.jo + R) &&
-                  !(__fadd_rn(rec_sq(a.x, gc[i]), rec_sq(a.y, gc[j])) > a.shell2);
+            a = A[l];
+            hs = !(i < a.io - R || i > a.io + R || je < a.jo - R || jb > a.jo + R);
+            he = a.reach_e >= 0 && !(i < a.iw - a.reach_e || i > a.iw + a.reach_e || je < a.jw - a.reach_e ||
+                                     jb > a.jw + a.reach_e);
         }
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (hit && out) out[base + n + __popc(m & ((1u << lane) - 1u))] = l;
-        n += __popc(m);
-    }
-    if (!out && lane == 0) cnt[row] = n;
-}
-
-__global__ void k_rec_shell(RecParams P, const RecAtom *__restrict__ A, const float *__restrict__ gc,
-                            const int *__restrict__ start, const int *__restrict__ list, float *__restrict__ grid) {
-    const int ng = P.ng;
-    const size_t ng3 = (size_t)ng * ng * ng;
-    const size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (c >= ng3) return;
-    const int i = (int)(c / ((size_t)ng * ng)), j = (int)((c / ng) % ng), k = (int)(c % ng);
-    const int row = i * ng + j, R = P.reach_shell;
-    float v = 0.f;
-    for (int e = start[row]; e < start[row + 1]; ++e) {
-        const RecAtom &a = A[list[e]];
-        if (k < a.ko - R || k > a.ko + R) continue;
-        const float d = __fadd_rn(__fadd_rn(rec_sq(a.x, gc[i]), rec_sq(a.y, gc[j])), rec_sq(a.z, gc[k]));
-        if (d < a.shell2) v = __double2float_rn(__dadd_rn((double)v, a.term));
-    }
-    if (grid[c] != P.eps_core) grid[c] = v;
-}
-
-// Charged atoms (in order) whose field cube reaches plane i: one warp per plane.
-__global__ void k_rec_planes(RecParams P, const RecAtom *__restrict__ A, int *__restrict__ cnt,
-                             const int *__restrict__ start, int *__restrict__ out) {
-    const int i = (int)((blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5);
-    const int lane = threadIdx.x & 31;
-    if (i >= P.ng) return;   // whole warps
-    int n = 0;
-    const int base = out ? start[i] : 0;
-    for (int l0 = 0; l0 < P.na; l0 += 32) {
-        const int l = l0 + lane;
-        bool hit = false;
-        if (l < P.na) {
-            const RecAtom &a = A[l];
-            hit = a.reach_e >= 0 && i >= a.iw - a.reach_e && i <= a.iw + a.reach_e;
+        const unsigned hit = __ballot_sync(0xffffffffu, hs || he);
+        if (lane == 0) wcount[warp] = __popc(hit);
+        __syncthreads();
+        int at = n, tot = 0;
+#pragma unroll
+        for (int w = 0; w < kRecRows; ++w) {
+            const int cw = wcount[w];
+            if (w < warp) at += cw;
+            tot += cw;
         }
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (hit && out) out[base + n + __popc(m & ((1u << lane) - 1u))] = l;
-        n += __popc(m);
-    }
-    if (!out && lane == 0) cnt[i] = n;
-}
-
-__global__ void k_rec_elec(RecParams P, const RecAtom *__restrict__ A, const float *__restrict__ gc,
-                           const int *__restrict__ start, const int *__restrict__ list,
-                           const float *__restrict__ grid_r, float *__restrict__ grid_i) {
-    const int ng = P.ng;
-    const size_t ng3 = (size_t)ng * ng * ng;
-    const size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (c >= ng3) return;
-    float v = 0.f;
-    if (!(grid_r[c] < 0.0f)) {   // receptor core cells carry no field
-        const int i = (int)(c / ((size_t)ng * ng)), j = (int)((c / ng) % ng), k = (int)(c % ng);
-        const float coef = __fmul_rn(P.e_ratio, -2800.0f);
-        for (int e = start[i]; e < start[i + 1]; ++e) {
-            const RecAtom &a = A[list[e]];
-            if (j < a.jw - a.reach_e || j > a.jw + a.reach_e || k < a.kw - a.reach_e || k > a.kw + a.reach_e)
-                continue;
-            const float d2 = __fadd_rn(rec_sq(a.x, gc[i]), rec_sq(a.y, gc[j]));
-            const float r = __fsqrt_rn(__fadd_rn(d2, rec_sq(a.z, gc[k])));
-            float eps;
-            if (r >= 8.0f) eps = 80.0f;
-            else if (r > 6.0f) eps = __fadd_rn(__fmul_rn(38.0f, r), -224.0f);
-            else eps = 4.0f;
-            v = __fadd_rn(v, __fdiv_rn(__fdiv_rn(__fmul_rn(coef, a.q), eps), r));
+        if (hs || he) {
+            RecEntry e;
+            e.x = a.x;
+            e.y = a.y;
+            e.z = a.z;
+            e.shell2 = hs ? a.shell2 : -1.f;
+            e.term = a.term;
+            e.cq = a.cq;
+            e.cq4 = __fdiv_rn(a.cq, 4.0f);
+            e.cq80 = __fdiv_rn(a.cq, 80.0f);
+            e.jo = a.jo;
+            e.ko = a.ko;
+            e.jw = a.jw;
+            e.kw = a.kw;
+            e.reach_e = he ? a.reach_e : -1;
+            list[at + __popc(hit & ((1u << lane) - 1u))] = e;
         }
+        n += tot;
+        __syncthreads();
+        if (n + NT <= kRecList && l0 + NT < P.na) continue;   // room for another step
+        if (j < ng) {
+            for (int f = 0; f < n; ++f) {
+                const RecEntry &e = list[f];
+                const float d2 = __fadd_rn(rec_sq(e.x, gi), rec_sq(e.y, gj));
+                const bool s = e.shell2 >= 0.f && j >= e.jo - R && j <= e.jo + R && !(d2 > e.shell2);
+                const int re = e.reach_e;
+                const bool q = re >= 0 && j >= e.jw - re && j <= e.jw + re;
+                if (!s && !q) continue;   // the whole warp
+#pragma unroll
+                for (int m = 0; m < KM; ++m) {
+                    const int k = lane + 32 * m;
+                    const bool sk = s && k >= e.ko - R && k <= e.ko + R;
+                    const bool qk = q && k >= e.kw - re && k <= e.kw + re;
+                    if (!__any_sync(0xffffffffu, sk || qk)) continue;
+                    const float d3 = __fadd_rn(d2, rec_sq(e.z, gk[m]));
+                    if (sk && d3 < e.shell2) shell[m] = __double2float_rn(__dadd_rn((double)shell[m], e.term));
+                    if (qk) {
+                        const float r = __fsqrt_rn(d3);
+                        float ce;
+                        if (r >= 8.0f) ce = e.cq80;
+                        else if (r > 6.0f) ce = __fdiv_rn(e.cq, __fadd_rn(__fmul_rn(38.0f, r), -224.0f));
+                        else ce = e.cq4;
+                        field[m] = __fadd_rn(field[m], __fdiv_rn(ce, r));
+                    }
+                }
+            }
+        }
+        n = 0;
+        __syncthreads();
     }
-    grid_i[c] = v;
+    if (j >= ng) return;
+#pragma unroll
+    for (int m = 0; m < KM; ++m) {
+        const int k = lane + 32 * m;
+        if (k >= ng) continue;
+        const unsigned long long cw = core[i * ng + j].w[k >> 6], ow = open[i * ng + j].w[k >> 6];
+        const bool is_open = (ow >> (k & 63)) & 1ull, is_core = (cw >> (k & 63)) & 1ull;
+        // cavities (neither core nor open) count as core; a core value equal
+        // to the open-space marker makes the core cells open (core_open)
+        const bool full = is_core ? !core_open : !is_open;
+        const float v = full ? P.eps_core : shell[m];
+        const size_t c = ((size_t)i * ng + j) * ng + k;
+        grid_r[c] = v;
+        grid_i[c] = v < 0.0f ? 0.f : field[m];   // receptor core cells carry no field
+    }
 }
 
 }  // namespace mdb
