@@ -567,7 +567,6 @@ __global__ void __launch_bounds__(kNT1, 1)
     constexpr int NG = N / 2, OFF = N / 4, PITCH = N + 1;
     constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
     constexpr int W = VoxShared<NG>::W;
-    constexpr bool PR = prune_ok<N>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *S = reinterpret_cast<float2 *>(smem_raw);   // N x PITCH
 
@@ -575,11 +574,6 @@ __global__ void __launch_bounds__(kNT1, 1)
     const int b = blockIdx.y;
     const int tid = threadIdx.x;
 
-    if constexpr (!PR && MODE != 2) {
-        // unpruned passes read the padding: make it zero
-        for (int c = tid; c < N * PITCH; c += blockDim.x) S[c] = make_float2(0.f, 0.f);
-        __syncthreads();
-    }
     if (MODE == 1) {
         for (int c = tid; c < NG * NG; c += blockDim.x) {
             const int q = c / NG, s = c % NG;
@@ -625,7 +619,7 @@ __global__ void __launch_bounds__(kNT1, 1)
     // z-FFT of the NG non-zero rows (lanes = rows, pruned columns)
     for (int it = tid; it < NG * R2; it += blockDim.x) {
         const int t = it / NG, q = it % NG;
-        fft_phase1<N, -1, PR>(S + (q + OFF) * PITCH, 1, t, G.tw);
+        padded_phase1<N>(S + (q + OFF) * PITCH, 1, t, G.tw);
     }
     __syncthreads();
     {
@@ -651,7 +645,7 @@ __global__ void __launch_bounds__(kNT1, 1)
     // y-FFT of all N columns (lanes = columns, pruned rows); phase 2 -> global
     for (int it = tid; it < N * R2; it += blockDim.x) {
         const int t = it / N, c = it % N;
-        fft_phase1<N, -1, PR>(S + c, PITCH, t, G.tw);
+        padded_phase1<N>(S + c, PITCH, t, G.tw);
     }
     __syncthreads();
     float2 *Ab = A + ((size_t)b * NG + p) * N * N;
@@ -715,17 +709,10 @@ __global__ void __launch_bounds__(kNT1B, fwd_cb_fits<N>() ? 2 : 1)
     constexpr int NG = N / 2, OFF = N / 4, PZ = N + 1, CB = fwd_cb_width<N>(), PB = CB + 1;
     constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
     constexpr int W = VoxShared<NG>::W;
-    constexpr bool PR = prune_ok<N>();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *Z = reinterpret_cast<float2 *>(smem_raw);   // NG rows x PZ
     float2 *Y = Z + NG * PZ;                             // N rows x PB
     const int p = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
-    if constexpr (!PR && MODE != 2) {
-        // the unpruned z pass reads the padding columns: make them zero
-        for (int c = tid; c < NG * PZ; c += blockDim.x) Z[c] = make_float2(0.f, 0.f);
-        __syncthreads();
-    }
-
     // the plane's NG rows at column offset OFF (the pruned passes read no
     // other column)
     if constexpr (MODE == 1) {
@@ -773,7 +760,7 @@ __global__ void __launch_bounds__(kNT1B, fwd_cb_fits<N>() ? 2 : 1)
     // z-FFT of the NG rows (lanes = rows, pruned columns)
     for (int it = tid; it < NG * R2; it += blockDim.x) {
         const int t = it / NG, q = it % NG;
-        fft_phase1<N, -1, PR>(Z + q * PZ, 1, t, G.tw);
+        padded_phase1<N>(Z + q * PZ, 1, t, G.tw);
     }
     __syncthreads();
     {
@@ -803,19 +790,7 @@ __global__ void __launch_bounds__(kNT1B, fwd_cb_fits<N>() ? 2 : 1)
             const int t = it / CB, c = it % CB;
             if (cb + c >= N) continue;
             float2 v[R1];
-            static_for<0, R1>([&](auto m_) {
-                constexpr int m = decltype(m_)::value;
-                if constexpr (PR) {
-                    if constexpr (m < R1 / 4 || m >= 3 * R1 / 4) {
-                        v[m] = make_float2(-0.f, -0.f);
-                    } else {
-                        v[m] = Z[(t + R2 * (m - R1 / 4)) * PZ + cb + c];   // row n - OFF, n = t + R2 m
-                    }
-                } else {
-                    const int q = t + R2 * m - OFF;   // resident row of y = t + R2 m, if any
-                    v[m] = ((unsigned)q < (unsigned)NG) ? Z[q * PZ + cb + c] : make_float2(0.f, 0.f);
-                }
-            });
+            padded_inputs<N, R1, R2>(v, t, [&](int q) { return Z[q * PZ + cb + c]; });   // resident row q
             Dft<R1, -1>::run(v);
             static_for<0, R1>([&](auto k1_) {
                 constexpr int k1 = decltype(k1_)::value;
@@ -848,20 +823,15 @@ __global__ void __launch_bounds__(kNT)
     constexpr int TILES = (N + kLT - 1) / kLT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2 *X = reinterpret_cast<float2 *>(smem_raw);   // N x kLT
-    constexpr bool PR = prune_ok<N>();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int ky = blockIdx.x / TILES;
     const int kz = (blockIdx.x % TILES) * kLT + lane;
     const bool ok = kz < N;
-    if constexpr (!PR) {
-        for (int c = threadIdx.x; c < N * kLT; c += blockDim.x) X[c] = make_float2(0.f, 0.f);
-        __syncthreads();
-    }
     for (int pp = warp; pp < NG; pp += nwarp)
         X[(pp + OFF) * kLT + lane] = ok ? A[((size_t)pp * N + ky) * N + kz] : make_float2(0.f, 0.f);
     __syncthreads();
     for (int it = threadIdx.x; it < kLT * R2; it += blockDim.x)
-        fft_phase1<N, -1, PR>(X + (it % kLT), kLT, it / kLT, G.tw);
+        padded_phase1<N>(X + (it % kLT), kLT, it / kLT, G.tw);
     __syncthreads();
     for (int it = threadIdx.x; it < kLT * R1; it += blockDim.x) {
         const int ln = it % kLT, u = it / kLT;

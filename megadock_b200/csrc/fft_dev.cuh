@@ -12,14 +12,11 @@
 // item, so the inter-phase twiddle index t*k1 is warp-uniform (broadcast load).
 //
 // Zero padding: docking grids carry data only in the middle half of each axis
-// ([N/4, 3N/4)).  With R1 % 4 == 0 the pruned phase 1 loads exactly
-// m in [R1/4, 3R1/4) for every t and skips the other (zero) inputs.  The
-// skipped inputs are -0: x + (-0) = x and (-0) - x = -x hold for every x, so
-// the compiler drops those adds from the codelet (with +0 it may not: +0 + -0
-// is +0); the outputs are the same bits (B200, N = 128: identical records).  When
-// N/2 is odd (N % 4 == 2) the data sit at [floor(N/4), floor(N/4) + N/2) and no
-// split prunes evenly: those sizes run the unpruned phase 1 over explicit zeros
-// (prune_ok<N>() false).
+// ([floor(N/4), floor(N/4) + N/2)), so half the inputs of a first pass are
+// known zeros (padded_inputs).  The skipped inputs are -0: x + (-0) = x and
+// (-0) - x = -x hold for every x, so the compiler drops those adds from the
+// codelet (with +0 it may not: +0 + -0 is +0); the outputs are the same bits
+// (B200, N = 128: identical records).
 //
 // The small DFTs are generated at compile time: prime radices 2, 3, 5, 7, 11
 // are direct DFTs (radix 4 is a butterfly); composite radices recurse through
@@ -220,9 +217,8 @@ struct Dft {
 };
 
 // ------------------------------------------------------------------ line plans
-// Supported FFT edge lengths and their split N = R1 * R2.  Edges that carry the
-// zero-padded ligand / receptor (N % 4 == 0) use R1 % 4 == 0 so the pruned
-// first pass works; the half edges of the complex-to-real pass need not.
+// Supported FFT edge lengths and their split N = R1 * R2 (R1 % 4 == 0 where N
+// allows it: no input of the first pass is then part padding, part data).
 template <int N>
 struct Plan;
 #define MDB_PLAN(N_, R1_, R2_)                                  \
@@ -353,13 +349,6 @@ MDB_PLAN(243, 9, 27)
 MDB_PLAN(245, 7, 35)
 #undef MDB_PLAN
 
-// Whether the first passes of an axis of length N can skip the zero padding
-// (data in the middle half, split with R1 % 4 == 0).
-template <int N>
-constexpr bool prune_ok() {
-    return N % 4 == 0 && Plan<N>::R1 % 4 == 0;
-}
-
 // Zero padding of input m of a radix-R1 first pass over stride R2 on an axis
 // of length N (data in [floor(N/4), floor(N/4) + N/2)): 0 = padding for every
 // item t < R2, 2 = data for every item, 1 = depends on the item.  With
@@ -387,30 +376,19 @@ __device__ __forceinline__ void padded_inputs(float2 (&v)[R1], int t, const Load
     });
 }
 
-// Phase 1 of one item on a line at `b` with element stride `es`.
-// tw: W_N^j = exp(-2*pi*i*j/N), j < N (forward table); S selects the sign.
-template <int N, int S, bool PRUNE>
-__device__ __forceinline__ void fft_phase1(float2 *b, int es, int t, const float2 *__restrict__ tw) {
+// Forward phase 1 of item t on a zero-padded line at `b` (axis position 0)
+// with element stride `es`, by the line plan of N; tw[j] = exp(-2 pi i j / N).
+// The padding is never read.
+template <int N>
+__device__ __forceinline__ void padded_phase1(float2 *b, int es, int t, const float2 *__restrict__ tw) {
     constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
-    static_assert(!PRUNE || R1 % 4 == 0, "pruned first pass needs R1 % 4 == 0");
     float2 v[R1];
-    static_for<0, R1>([&](auto m_) {
-        constexpr int m = decltype(m_)::value;
-        if constexpr (PRUNE && (m < R1 / 4 || m >= 3 * R1 / 4)) {
-            v[m] = make_float2(-0.f, -0.f);
-        } else {
-            v[m] = b[(t + R2 * m) * es];
-        }
-    });
-    Dft<R1, S>::run(v);
+    padded_inputs<N, R1, R2>(v, t, [&](int y) { return b[(y + N / 4) * es]; });
+    Dft<R1, -1>::run(v);
     static_for<0, R1>([&](auto k1_) {
         constexpr int k1 = decltype(k1_)::value;
         float2 x = v[k1];
-        if constexpr (k1 != 0) {
-            float2 w = __ldg(&tw[t * k1]);
-            if (S > 0) w.y = -w.y;
-            x = cmul(x, w);
-        }
+        if constexpr (k1 != 0) x = cmul(x, __ldg(&tw[t * k1]));
         b[(k1 * R2 + t) * es] = x;
     });
 }
