@@ -1125,6 +1125,22 @@ __global__ void __launch_bounds__(XPlan<N>::NT, XPlan<N>::OCC)
     }
 }
 
+// Inverse plane kernels: one thread asks for the rows its CTA's place will need
+// one wave of CTAs later to be brought into L2, so that wave's first loads do
+// not wait for DRAM.  Worth it where a wave of planes (a few hundred, 64 to 200
+// KB each) sits in L2 beside the running one: N = 128 3.31 -> 3.15 us per
+// rotation, 144 5.73 -> 5.51, 160 8.12 -> 7.69, 216 29.8 -> 28.5; 96 and 108
+// equal, 256 and 330 1.5 % slower (B200).
+constexpr int kSMs = 148;
+template <int N>
+constexpr bool inv_prefetch() {
+    return N > 112 && N <= 224;
+}
+// bytes and the address are multiples of 16 (N is even)
+__device__ __forceinline__ void prefetch_l2(const void *p, unsigned bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // ------------------------------------------------------------------ K3
 // Selection order for top-t: larger key first, then smaller linear index.
 // NaN keys are never selected (they fail every comparison in the reference).
@@ -1408,6 +1424,10 @@ __global__ void __launch_bounds__(kNT, c2r_min_blocks<N, V>())
     const int b = blockIdx.y;
     const int tid = threadIdx.x;
     const float2 *Gp = Gh + ((size_t)b * N + x) * NH * N;
+    if constexpr (inv_prefetch<N>()) {
+        const unsigned next = blockIdx.y * N + blockIdx.x + kSMs * c2r_min_blocks<N, V>();
+        if (tid == 0 && next < gridDim.y * N) prefetch_l2(Gh + (size_t)next * NH * N, NH * N * sizeof(float2));
+    }
 
     // The z pass works on whole rows: warp w owns rows [w NH/16, (w+1) NH/16) in
     // both of its passes, so the passes are separated by warp barriers only; the

@@ -56,6 +56,11 @@ __global__ void __cluster_dims__(P::C, 1, 1) __launch_bounds__(P::NT, P::OCC)
     const int x = blockIdx.x / C, rank = blockIdx.x % C, b = blockIdx.y, tid = threadIdx.x;
     const float2 *Gp = Gh + (((size_t)b * N + x) * NH + (size_t)rank * RB) * N;
     const int rows = min(RB, NH - rank * RB);
+    if constexpr (inv_prefetch<N>()) {   // the same rows of the plane one wave ahead
+        const unsigned next = blockIdx.y * N + x + (kSMs * P::OCC + C - 1) / C;
+        if (tid == 0 && rows > 0 && next < gridDim.y * N)
+            prefetch_l2(Gh + ((size_t)next * NH + (size_t)rank * RB) * N, rows * N * (unsigned)sizeof(float2));
+    }
     // (1a) inverse kz pass 1 of this CTA's rows, straight from global
     for (int it = tid; it < rows * R2; it += NT) {
         const int row = it / R2, tt = it % R2;
