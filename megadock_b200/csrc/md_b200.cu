@@ -697,12 +697,13 @@ int adjoint_core(md_ctx *ctx, const float *rotmat, int n, const int4 *shift, con
     const int B = group_of(ctx, n, 1);
     int rc = ensure_work(ctx, B, 1);
     if (rc) return rc;
-    const size_t sz[8] = {sizeof(float) * 9 * n,       sizeof(float) * n,
+    const size_t sz[9] = {sizeof(float) * 9 * n,       sizeof(float) * n,
                           sizeof(int4) * n,            sizeof(float) * 2 * ng3,
                           sizeof(float) * 2 * ng3 * B, sizeof(float) * std::max(ctx->na, 1),
-                          sizeof(int) * std::max(n_lig, 1), sizeof(float) * 2 * ng3 * std::max(n_lig, 0)};
-    char *p[8];
-    if ((rc = carve_scratch(ctx, sz, 8, p))) return rc;
+                          sizeof(int) * std::max(n_lig, 1), sizeof(float) * 2 * ng3 * std::max(n_lig, 0),
+                          sizeof(double) * kAdjBlocks};
+    char *p[9];
+    if ((rc = carve_scratch(ctx, sz, 9, p))) return rc;
     float *d_rot = reinterpret_cast<float *>(p[0]), *d_w = reinterpret_cast<float *>(p[1]);
     int4 *d_shift = reinterpret_cast<int4 *>(p[2]);
     float *d_grad = reinterpret_cast<float *>(p[3]), *d_vox = reinterpret_cast<float *>(p[4]);
@@ -740,14 +741,13 @@ int adjoint_core(md_ctx *ctx, const float *rotmat, int n, const int4 *shift, con
         k_adj_ligand<<<dim3(blocks, n_lig), thr, 0, s>>>(N, ng, n_lig, d_sel, ctx->d_recv, ctx->d_recv + ng3,
                                                          d_shift, d_w, d_lg, d_lg + ng3 * n_lig);
     }
+    // the receptor's imaginary grid is alpha times a fixed-support unit grid
+    double *d_part = reinterpret_cast<double *>(p[8]), part[kAdjBlocks];
+    if (d_alpha) k_adj_dot<<<kAdjBlocks, 256, 0, s>>>(ng3, d_grad + ng3, ctx->d_recv + ng3, d_part);
     step(cudaGetLastError());
-    std::vector<float> gi(d_alpha ? ng3 : 0), ri(d_alpha ? ng3 : 0);
     if (d_rec_r) step(cudaMemcpyAsync(d_rec_r, d_grad, sizeof(float) * ng3, cudaMemcpyDeviceToHost, s));
     if (d_rec_i) step(cudaMemcpyAsync(d_rec_i, d_grad + ng3, sizeof(float) * ng3, cudaMemcpyDeviceToHost, s));
-    if (d_alpha) {
-        step(cudaMemcpyAsync(gi.data(), d_grad + ng3, sizeof(float) * ng3, cudaMemcpyDeviceToHost, s));
-        step(cudaMemcpyAsync(ri.data(), ctx->d_recv + ng3, sizeof(float) * ng3, cudaMemcpyDeviceToHost, s));
-    }
+    if (d_alpha) step(cudaMemcpyAsync(part, d_part, sizeof(part), cudaMemcpyDeviceToHost, s));
     if (d_charge) step(cudaMemcpyAsync(d_charge, d_dq, sizeof(float) * ctx->na, cudaMemcpyDeviceToHost, s));
     if (n_lig > 0) {
         step(cudaMemcpyAsync(d_lig_r, d_lg, sizeof(float) * ng3 * n_lig, cudaMemcpyDeviceToHost, s));
@@ -759,9 +759,8 @@ int adjoint_core(md_ctx *ctx, const float *rotmat, int n, const int4 *shift, con
         return MD_ERR_CUDA;
     }
     if (d_alpha) {
-        // the receptor's imaginary grid is alpha times a fixed-support unit grid
         double acc = 0.0;
-        for (size_t x = 0; x < ng3; ++x) acc += (double)gi[x] * (double)ri[x];
+        for (double v : part) acc += v;
         *d_alpha = alpha != 0.f ? acc / alpha : std::nan("");
     }
     return MD_OK;
