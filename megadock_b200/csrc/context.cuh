@@ -171,13 +171,11 @@ struct Sized {
     }
     template <int MODE>
     static void plane_fwd(cudaStream_t s, int nb, const LigandView &L, const GridView &G, const uint32_t *vbits,
-                          const int2 *qlist, const int *qcount, const float *sr, const float *si, float2 *A,
-                          float *vr, float *vi) {
+                          const int2 *qlist, const int *qcount, const float *sr, const float *si, float2 *A) {
         if constexpr (use_cb<MODE>())
-            k_plane_fwd_cb<N, MODE><<<dim3(NG, nb), kNT1B, fwd_cb_smem<N>(), s>>>(L, G, vbits, qlist, qcount, sr, si,
-                                                                                   A, vr, vi);
+            k_plane_fwd_cb<N, MODE><<<dim3(NG, nb), kNT1B, fwd_cb_smem<N>(), s>>>(L, G, vbits, qlist, qcount, sr, si, A);
         else
-            k_plane_fwd<N, MODE><<<dim3(NG, nb), kNT1, smem_fwd(), s>>>(L, G, vbits, qlist, qcount, sr, si, A, vr, vi);
+            k_plane_fwd<N, MODE><<<dim3(NG, nb), kNT1, smem_fwd(), s>>>(L, G, vbits, qlist, qcount, sr, si, A);
     }
 
     static cudaError_t set_attrs() {
@@ -190,12 +188,10 @@ struct Sized {
         if constexpr (kStaged) {
             set((const void *)k_rows_fwd<N, 0>, rows_smem<N>());
             set((const void *)k_rows_fwd<N, 1>, rows_smem<N>());
-            set((const void *)k_rows_fwd<N, 2>, rows_smem<N>());
             set((const void *)k_cols_fwd<N>, cols_fwd_smem(N));
         } else {
             set_fwd<0>(set);
             set_fwd<1>(set);
-            set_fwd<2>(set);
         }
         if (e == cudaSuccess) e = set_inv_attrs<N>();
         set((const void *)k_xline_rec<N>, smem_xrec());
@@ -206,28 +202,26 @@ struct Sized {
         return e;
     }
 
-    // Forward plane transforms of nb rotations (MODE 0/1) or the voxel planes
-    // themselves (MODE 2) in the staged form: row launch, then column launch.
+    // Forward plane transforms of nb rotations in the staged form: row launch,
+    // then column launch.
     template <int MODE>
     static void staged_fwd(cudaStream_t s, int nb, const LigandView &L, const GridView &G, const uint32_t *vbits,
-                           const int2 *qlist, const int *qcount, const float *sr, const float *si, float2 *A,
-                           float *vr, float *vi) {
+                           const int2 *qlist, const int *qcount, const float *sr, const float *si, float2 *A) {
         k_rows_fwd<N, MODE><<<dim3(NG, (NG + kRB - 1) / kRB, nb), kNTS, rows_smem<N>(), s>>>(L, G, vbits, qlist, qcount,
-                                                                                           sr, si, A, vr, vi);
-        if constexpr (MODE != 2) k_cols_fwd<N><<<dim3(NG, (N + kCB - 1) / kCB, nb), kNTS, cols_fwd_smem(N), s>>>(G, A);
+                                                                                           sr, si, A);
+        k_cols_fwd<N><<<dim3(NG, (N + kCB - 1) / kCB, nb), kNTS, cols_fwd_smem(N), s>>>(G, A);
     }
     template <int MODE>
     static void any_fwd(cudaStream_t s, int nb, const LigandView &L, const GridView &G, const uint32_t *vbits,
-                        const int2 *qlist, const int *qcount, const float *sr, const float *si, float2 *A, float *vr,
-                        float *vi) {
-        if constexpr (kStaged) staged_fwd<MODE>(s, nb, L, G, vbits, qlist, qcount, sr, si, A, vr, vi);
-        else plane_fwd<MODE>(s, nb, L, G, vbits, qlist, qcount, sr, si, A, vr, vi);
+                        const int2 *qlist, const int *qcount, const float *sr, const float *si, float2 *A) {
+        if constexpr (kStaged) staged_fwd<MODE>(s, nb, L, G, vbits, qlist, qcount, sr, si, A);
+        else plane_fwd<MODE>(s, nb, L, G, vbits, qlist, qcount, sr, si, A);
     }
 
     static void receptor(md_ctx *c, const float *d_r, const float *d_i) {
         GridView G{c->ng, c->gw, 0.f, c->d_gc, c->d_tw};
         LigandView L{0, nullptr, nullptr, 1.f};
-        any_fwd<1>(c->stream, 1, L, G, nullptr, nullptr, nullptr, d_r, d_i, c->ws[0].A, nullptr, nullptr);
+        any_fwd<1>(c->stream, 1, L, G, nullptr, nullptr, nullptr, d_r, d_i, c->ws[0].A);
         k_xline_rec<N><<<dim3(N * TILES, 1), kNT, smem_xrec(), c->stream>>>(G, c->ws[0].A, c->d_Rh);
     }
 
@@ -248,7 +242,7 @@ struct Sized {
         LigandView L{c->na, c->d_atom, c->d_rad2, c->delta};
         const WorkSet &w = c->ws[0];
         voxelize(c, w, d_rot9, nb, c->stream);
-        any_fwd<2>(c->stream, nb, L, G, w.vbits, w.qlist, w.qcount, nullptr, nullptr, nullptr, d_vr, d_vi);
+        k_vox_store<NG><<<dim3(NG, nb), kNT0, 0, c->stream>>>(L, w.vbits, w.qlist, w.qcount, d_vr, d_vi);
     }
 
     static void voxels(md_ctx *c, const float *d_rot9, float *d_vr, float *d_vi) {
@@ -256,7 +250,7 @@ struct Sized {
         LigandView L{c->na, c->d_atom, c->d_rad2, c->delta};
         const WorkSet &w = c->ws[0];
         voxelize(c, w, d_rot9, 1, c->stream);
-        any_fwd<2>(c->stream, 1, L, G, w.vbits, w.qlist, w.qcount, nullptr, nullptr, nullptr, d_vr, d_vi);
+        k_vox_store<NG><<<dim3(NG, 1), kNT0, 0, c->stream>>>(L, w.vbits, w.qlist, w.qcount, d_vr, d_vi);
     }
 
     // One launch group: nb rotations whose matrices start at d_rot9, on work
@@ -269,7 +263,7 @@ struct Sized {
         const float nf3f = (float)((long long)N * N * N);
         voxelize(c, w, d_rot9, nb, s);
         if (ev) cudaEventRecord(ev[1], s);
-        any_fwd<0>(s, nb, L, G, w.vbits, w.qlist, w.qcount, nullptr, nullptr, w.A, nullptr, nullptr);
+        any_fwd<0>(s, nb, L, G, w.vbits, w.qlist, w.qcount, nullptr, nullptr, w.A);
         if (ev) cudaEventRecord(ev[2], s);
         k_xline_fold<N><<<xline_grid<N>(nb), XPlan<N>::NT, xline_smem<N>(), s>>>(G, w.A, c->d_Rh, w.G);
         if (ev) cudaEventRecord(ev[3], s);

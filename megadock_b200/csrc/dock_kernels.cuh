@@ -554,16 +554,47 @@ __global__ void __launch_bounds__(kNT0)
     if (tid == 0) qcount[(size_t)b * NG + p] = count;
 }
 
+// The voxel grids themselves ([nb][NG^3] real, imaginary) from K0's bit planes
+// and charge lists, for the adjoint and the direct pose scores: CTA = (x-plane,
+// rotation), the plane written once, then its charged cells.  Bound by the
+// stores.  The forward plane kernel without its FFT did this through a
+// shared-memory plane, one CTA per SM (64 rotations at N = 96 42.8 us); the
+// adjoint of 3,600 rotations there, nineteen such chunks, went 1.95 -> 1.78 ms
+// (B200).
+template <int NG>
+__global__ void __launch_bounds__(kNT0)
+    k_vox_store(LigandView L, const uint32_t *__restrict__ vbits, const int2 *__restrict__ qlist,
+                const int *__restrict__ qcount, float *__restrict__ vox_r, float *__restrict__ vox_i) {
+    constexpr int W = VoxShared<NG>::W;
+    const int p = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+    const size_t plane = (size_t)b * NG + p;
+    const uint32_t *vb = vbits + plane * 2 * NG * W;
+    float *vr = vox_r + plane * NG * NG, *vi = vox_i + plane * NG * NG;
+#pragma unroll 4
+    for (int c = tid; c < NG * NG; c += kNT0) {
+        const int q = c / NG, s = c % NG;
+        const uint32_t bit = 1u << (s & 31);
+        const uint32_t w2 = __ldg(&vb[q * W + (s >> 5)]), w1 = __ldg(&vb[NG * W + q * W + (s >> 5)]);
+        vr[c] = (w2 & bit) ? L.delta : (w1 & bit) ? 1.0f : 0.0f;
+        vi[c] = 0.f;
+    }
+    __syncthreads();   // the zeros before the charges
+    const int nq = qcount[plane];
+    const int2 *ql = qlist + plane * NG * NG;
+    for (int e = tid; e < nq; e += kNT0) {
+        const int2 c = ql[e];
+        vi[c.x] = __int_as_float(c.y);
+    }
+}
+
 // ------------------------------------------------------------------ K1
 // MODE 0: real part from the K0 bit planes + K0 charge list, store spectrum planes A.
 // MODE 1: receptor grids (re, im) loaded from global, store spectrum planes A.
-// MODE 2: like MODE 0 but store the voxel plane itself (ng x ng real and
-//         imaginary parts) for parity checks; no FFT.
 template <int N, int MODE>
 __global__ void __launch_bounds__(kNT1, 1)
     k_plane_fwd(LigandView L, GridView G, const uint32_t *__restrict__ vbits, const int2 *__restrict__ qlist,
                 const int *__restrict__ qcount, const float *__restrict__ src_r, const float *__restrict__ src_i,
-                float2 *__restrict__ A, float *__restrict__ vox_r, float *__restrict__ vox_i) {
+                float2 *__restrict__ A) {
     constexpr int NG = N / 2, OFF = N / 4, PITCH = N + 1;
     constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
     constexpr int W = VoxShared<NG>::W;
@@ -604,16 +635,6 @@ __global__ void __launch_bounds__(kNT1, 1)
             S[(c.x / NG + OFF) * PITCH + c.x % NG + OFF].y = __int_as_float(c.y);
         }
         __syncthreads();
-        if (MODE == 2) {
-            for (int c = tid; c < NG * NG; c += blockDim.x) {
-                const int q = c / NG, s = c % NG;
-                const float2 v = S[(q + OFF) * PITCH + s + OFF];
-                const size_t gidx = (((size_t)b * NG + p) * NG + q) * NG + s;
-                vox_r[gidx] = v.x;
-                vox_i[gidx] = v.y;
-            }
-            return;
-        }
     }
 
     // z-FFT of the NG non-zero rows (lanes = rows, pruned columns)
@@ -699,13 +720,12 @@ constexpr bool fwd_full_fits() {
     return (size_t)N * (N + 1) * sizeof(float2) <= kSmemMax;
 }
 
-// MODE as in k_plane_fwd: 0 ligand bits + charges, 1 receptor grids from
-// global, 2 the voxel plane itself (no FFT).
+// MODE as in k_plane_fwd: 0 ligand bits + charges, 1 receptor grids from global.
 template <int N, int MODE = 0>
 __global__ void __launch_bounds__(kNT1B, fwd_cb_fits<N>() ? 2 : 1)
     k_plane_fwd_cb(LigandView L, GridView G, const uint32_t *__restrict__ vbits, const int2 *__restrict__ qlist,
                    const int *__restrict__ qcount, const float *__restrict__ src_r, const float *__restrict__ src_i,
-                   float2 *__restrict__ A, float *__restrict__ vox_r, float *__restrict__ vox_i) {
+                   float2 *__restrict__ A) {
     constexpr int NG = N / 2, OFF = N / 4, PZ = N + 1, CB = fwd_cb_width<N>(), PB = CB + 1;
     constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2;
     constexpr int W = VoxShared<NG>::W;
@@ -746,16 +766,6 @@ __global__ void __launch_bounds__(kNT1B, fwd_cb_fits<N>() ? 2 : 1)
             Z[(c.x / NG) * PZ + c.x % NG + OFF].y = __int_as_float(c.y);
         }
         __syncthreads();
-        if constexpr (MODE == 2) {
-            for (int c = tid; c < NG * NG; c += blockDim.x) {
-                const int q = c / NG, s = c % NG;
-                const float2 v = Z[q * PZ + s + OFF];
-                const size_t gidx = (((size_t)b * NG + p) * NG + q) * NG + s;
-                vox_r[gidx] = v.x;
-                vox_i[gidx] = v.y;
-            }
-            return;
-        }
     }
     // z-FFT of the NG rows (lanes = rows, pruned columns)
     for (int it = tid; it < NG * R2; it += blockDim.x) {

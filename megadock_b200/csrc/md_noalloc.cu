@@ -152,8 +152,7 @@ void run_rotation(cudaStream_t s, const LigandView &L, const GridView &G, const 
     k_atom_prep<NG><<<1, nt, prep_smem<NG>(nt), s>>>(L, G, rot9, pr.srec, pr.sstart, pr.cq, pr.cstart);
     k_vox_bits<NG><<<dim3(NG, 1), kNT0, vox_bits_smem<NG>(), s>>>(L, G, pr.srec, pr.sstart, pr.cq, pr.cstart, vbits,
                                                                  qlist, qcount);
-    k_plane_fwd<N, 0><<<dim3(NG, 1), kNT1, Smem<N>::fwd(), s>>>(L, G, vbits, qlist, qcount, nullptr, nullptr, A,
-                                                               nullptr, nullptr);
+    k_plane_fwd<N, 0><<<dim3(NG, 1), kNT1, Smem<N>::fwd(), s>>>(L, G, vbits, qlist, qcount, nullptr, nullptr, A);
     k_xline_fold<N><<<xline_grid<N>(1), XPlan<N>::NT, Smem<N>::xline(), s>>>(G, A, Rh, Gsp);
     static_assert(inv_groups<N>() <= N * kMaxNoallocCluster, "candidate scratch");
     launch_inv<N>(s, G, Gsp, 1, t, 0, cand);

@@ -3,9 +3,8 @@
 // forward plane transform by separate launches through global memory:
 //
 //   K1r k_rows_fwd   (x-plane p, block of RB voxel rows): build the rows of
-//                    the voxel plane (ligand classes + ordered charge sums,
-//                    the receptor grids, or -- MODE 2 -- just store them) and
-//                    run the pruned forward z-FFT of each row into A[p][y][kz]
+//                    the voxel plane (ligand classes + ordered charge sums, or
+//                    the receptor grids) and run the pruned forward z-FFT of each row into A[p][y][kz]
 //                    for the NG data rows y;
 //   K1c k_cols_fwd   (x-plane p, block of CB columns kz): pruned forward y-FFT
 //                    of the columns, in place in A -> A[p][ky][kz].
@@ -47,13 +46,12 @@ constexpr size_t cols_fwd_smem(int N) { return (size_t)N * (kCB + 1) * sizeof(fl
 
 // K1r.  Grid (NG planes, ceil(NG / RB) row blocks, nb), kNTS threads.
 // MODE 0: ligand classes (K0 bit planes) and charged cells; MODE 1: receptor
-// grids src_r / src_i ([NG][NG][NG] floats); MODE 2: store the voxel rows to
-// vox_r / vox_i, no FFT.
+// grids src_r / src_i ([NG][NG][NG] floats).
 template <int N, int MODE>
 __global__ void __launch_bounds__(kNTS)
     k_rows_fwd(LigandView L, GridView G, const uint32_t *__restrict__ vbits, const int2 *__restrict__ qlist,
                const int *__restrict__ qcount, const float *__restrict__ src_r, const float *__restrict__ src_i,
-               float2 *__restrict__ A, float *__restrict__ vox_r, float *__restrict__ vox_i) {
+               float2 *__restrict__ A) {
     constexpr int NG = N / 2, OFF = N / 4;
     constexpr int R1 = RowPlan<N>::R1, R2 = RowPlan<N>::R2, STR = RowPlan<N>::STR, PZ = RowPlan<N>::PZ;
     constexpr int W = VoxShared<NG>::W;
@@ -98,16 +96,6 @@ __global__ void __launch_bounds__(kNTS)
             if ((unsigned)r < (unsigned)nr) at(r, c.x % NG).y = __int_as_float(c.y);
         }
         __syncthreads();
-        if constexpr (MODE == 2) {
-            for (int c = tid; c < nr * NG; c += kNTS) {
-                const int r = c / NG, s = c % NG;
-                const float2 v = at(r, s);
-                const size_t gidx = (((size_t)b * NG + p) * NG + q0 + r) * NG + s;
-                vox_r[gidx] = v.x;
-                vox_i[gidx] = v.y;
-            }
-            return;
-        }
     }
     // z-FFT of the block's rows: phase 1 in place, phase 2 to global (row y = q + OFF)
     for (int it = tid; it < nr * R2; it += kNTS) {
