@@ -281,17 +281,26 @@ __global__ void k_rec_apply(RecParams P, const RowMask<WORDS> *__restrict__ core
 
 // The two grids.  CTA = (i, kRecRows rows j), a warp per row, lane = k modulo
 // 32 with KM = ceil(ng / 32) cells each.  The atoms are walked once, in order:
-// the CTA collects those whose shell or field cube touches its rows into a
-// shared list (ballot compaction keeps the order), then every warp adds the
-// listed atoms' terms to its cells from registers.
+// the CTA collects those whose shell sphere or field cube touches its rows into
+// two shared lists (ballot compaction keeps the order), then every warp adds
+// the listed atoms' terms to its cells from registers.
+//
+// Bound by the field terms' issue (a square root and a division per cell of
+// every charged atom's cube).  The whole build with 3,661 atoms at ng = 64 takes
+// 1.03 ms on the B200 (1.36 with one list of both kinds and the shell's whole
+// search cube, 0.81 of it here).
 constexpr int kRecRows = 8;
 constexpr int kRecList = 512;
 
-struct RecEntry {
-    float x, y, z, shell2;   // shell2 < 0: the atom's shell cube misses this CTA
+struct RecShell {
     double term;
-    float cq, cq4, cq80;     // e_ratio -2800 q, over 4 and over 80 (the two constant dielectrics)
-    int jo, ko, jw, kw, reach_e;   // reach_e < 0: no field here
+    float x, y, z, shell2;
+    int jo, ko;
+};
+struct RecField {
+    float x, y, z;
+    float cq, cq4, cq80;   // e_ratio -2800 q, over 4 and over 80 (the two constant dielectrics)
+    int jw, kw, reach;
 };
 
 template <int WORDS, int KM>
@@ -300,13 +309,19 @@ __global__ void __launch_bounds__(32 * kRecRows)
                 const RowMask<WORDS> *__restrict__ core, const RowMask<WORDS> *__restrict__ open, int core_open,
                 float *__restrict__ grid_r, float *__restrict__ grid_i) {
     constexpr int NT = 32 * kRecRows;
-    __shared__ RecEntry list[kRecList];
-    __shared__ int wcount[kRecRows];
+    __shared__ RecShell shells[kRecList];
+    __shared__ RecField fields[kRecList];
+    __shared__ int2 wcount[kRecRows];
     const int ng = P.ng, i = blockIdx.x, jb = blockIdx.y * kRecRows;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int j = jb + warp, je = min(jb + kRecRows, ng) - 1;
     const int R = P.reach_shell;
     const float gi = gc[i], gj = gc[min(j, ng - 1)];
+    float glo = gc[jb], ghi = glo;   // the rows' coordinates lie between
+    for (int r = jb + 1; r <= je; ++r) {
+        glo = fminf(glo, gc[r]);
+        ghi = fmaxf(ghi, gc[r]);
+    }
     float gk[KM], shell[KM], field[KM];
 #pragma unroll
     for (int m = 0; m < KM; ++m) {
@@ -314,75 +329,74 @@ __global__ void __launch_bounds__(32 * kRecRows)
         shell[m] = 0.f;
         field[m] = 0.f;
     }
-    int n = 0;   // entries in the list (the same in every thread)
+    int ns = 0, nf = 0;   // entries in the lists (the same in every thread)
     for (int l0 = 0; l0 < P.na; l0 += NT) {
         const int l = l0 + tid;
-        bool hs = false, he = false;
+        bool hs = false, hf = false;
         RecAtom a;
         if (l < P.na) {
             a = A[l];
-            hs = !(i < a.io - R || i > a.io + R || je < a.jo - R || jb > a.jo + R);
-            he = a.reach_e >= 0 && !(i < a.iw - a.reach_e || i > a.iw + a.reach_e || je < a.jw - a.reach_e ||
+            // rounding is monotone, so a squared x or y distance above shell2
+            // keeps every rounded sum with it above too
+            hs = !(i < a.io - R || i > a.io + R || je < a.jo - R || jb > a.jo + R) && !(rec_sq(a.x, gi) > a.shell2) &&
+                 !(a.y < glo && rec_sq(a.y, glo) > a.shell2) && !(a.y > ghi && rec_sq(a.y, ghi) > a.shell2);
+            hf = a.reach_e >= 0 && !(i < a.iw - a.reach_e || i > a.iw + a.reach_e || je < a.jw - a.reach_e ||
                                      jb > a.jw + a.reach_e);
         }
-        const unsigned hit = __ballot_sync(0xffffffffu, hs || he);
-        if (lane == 0) wcount[warp] = __popc(hit);
+        const unsigned ms = __ballot_sync(0xffffffffu, hs), mf = __ballot_sync(0xffffffffu, hf);
+        if (lane == 0) wcount[warp] = make_int2(__popc(ms), __popc(mf));
         __syncthreads();
-        int at = n, tot = 0;
+        int as = ns, af = nf;
 #pragma unroll
         for (int w = 0; w < kRecRows; ++w) {
-            const int cw = wcount[w];
-            if (w < warp) at += cw;
-            tot += cw;
+            const int2 c = wcount[w];
+            if (w < warp) {
+                as += c.x;
+                af += c.y;
+            }
+            ns += c.x;
+            nf += c.y;
         }
-        if (hs || he) {
-            RecEntry e;
-            e.x = a.x;
-            e.y = a.y;
-            e.z = a.z;
-            e.shell2 = hs ? a.shell2 : -1.f;
-            e.term = a.term;
-            e.cq = a.cq;
-            e.cq4 = __fdiv_rn(a.cq, 4.0f);
-            e.cq80 = __fdiv_rn(a.cq, 80.0f);
-            e.jo = a.jo;
-            e.ko = a.ko;
-            e.jw = a.jw;
-            e.kw = a.kw;
-            e.reach_e = he ? a.reach_e : -1;
-            list[at + __popc(hit & ((1u << lane) - 1u))] = e;
-        }
-        n += tot;
+        const unsigned below = (1u << lane) - 1u;
+        if (hs) shells[as + __popc(ms & below)] = RecShell{a.term, a.x, a.y, a.z, a.shell2, a.jo, a.ko};
+        if (hf)
+            fields[af + __popc(mf & below)] = RecField{a.x,  a.y,  a.z,  a.cq,     __fdiv_rn(a.cq, 4.0f),
+                                                       __fdiv_rn(a.cq, 80.0f), a.jw, a.kw, a.reach_e};
         __syncthreads();
-        if (n + NT <= kRecList && l0 + NT < P.na) continue;   // room for another step
+        if (max(ns, nf) + NT <= kRecList && l0 + NT < P.na) continue;   // room for another step
         if (j < ng) {
-            for (int f = 0; f < n; ++f) {
-                const RecEntry &e = list[f];
+            for (int f = 0; f < ns; ++f) {
+                const RecShell &e = shells[f];
                 const float d2 = __fadd_rn(rec_sq(e.x, gi), rec_sq(e.y, gj));
-                const bool s = e.shell2 >= 0.f && j >= e.jo - R && j <= e.jo + R && !(d2 > e.shell2);
-                const int re = e.reach_e;
-                const bool q = re >= 0 && j >= e.jw - re && j <= e.jw + re;
-                if (!s && !q) continue;   // the whole warp
+                if (j < e.jo - R || j > e.jo + R || d2 > e.shell2) continue;   // the whole warp
 #pragma unroll
                 for (int m = 0; m < KM; ++m) {
                     const int k = lane + 32 * m;
-                    const bool sk = s && k >= e.ko - R && k <= e.ko + R;
-                    const bool qk = q && k >= e.kw - re && k <= e.kw + re;
-                    if (!__any_sync(0xffffffffu, sk || qk)) continue;
                     const float d3 = __fadd_rn(d2, rec_sq(e.z, gk[m]));
-                    if (sk && d3 < e.shell2) shell[m] = __double2float_rn(__dadd_rn((double)shell[m], e.term));
-                    if (qk) {
-                        const float r = __fsqrt_rn(d3);
-                        float ce;
-                        if (r >= 8.0f) ce = e.cq80;
-                        else if (r > 6.0f) ce = __fdiv_rn(e.cq, __fadd_rn(__fmul_rn(38.0f, r), -224.0f));
-                        else ce = e.cq4;
-                        field[m] = __fadd_rn(field[m], __fdiv_rn(ce, r));
-                    }
+                    if (d3 < e.shell2 && k >= e.ko - R && k <= e.ko + R)
+                        shell[m] = __double2float_rn(__dadd_rn((double)shell[m], e.term));
+                }
+            }
+            for (int f = 0; f < nf; ++f) {
+                const RecField &e = fields[f];
+                const int re = e.reach, k0 = e.kw - re, k1 = e.kw + re;
+                if (j < e.jw - re || j > e.jw + re) continue;   // the whole warp
+                const float d2 = __fadd_rn(rec_sq(e.x, gi), rec_sq(e.y, gj));
+#pragma unroll
+                for (int m = 0; m < KM; ++m) {
+                    if (32 * m > k1 || 32 * m + 31 < k0) continue;
+                    const int k = lane + 32 * m;
+                    if (k < k0 || k > k1) continue;
+                    const float r = __fsqrt_rn(__fadd_rn(d2, rec_sq(e.z, gk[m])));
+                    float ce;
+                    if (r >= 8.0f) ce = e.cq80;
+                    else if (r > 6.0f) ce = __fdiv_rn(e.cq, __fadd_rn(__fmul_rn(38.0f, r), -224.0f));
+                    else ce = e.cq4;
+                    field[m] = __fadd_rn(field[m], __fdiv_rn(ce, r));
                 }
             }
         }
-        n = 0;
+        ns = nf = 0;
         __syncthreads();
     }
     if (j >= ng) return;
