@@ -166,13 +166,17 @@ struct Sized {
     }
     template <int MODE, class Set>
     static void set_fwd(Set &set) {
-        if constexpr (use_cb<MODE>()) set((const void *)k_plane_fwd_cb<N, MODE>, fwd_cb_smem<N>());
+        if constexpr (fwd_pipe<N>()) set((const void *)k_plane_fwd_pipe<N, MODE>, FwdPipe<N>::bytes);
+        else if constexpr (use_cb<MODE>()) set((const void *)k_plane_fwd_cb<N, MODE>, fwd_cb_smem<N>());
         else set((const void *)k_plane_fwd<N, MODE>, smem_fwd());
     }
     template <int MODE>
     static void plane_fwd(cudaStream_t s, int nb, const LigandView &L, const GridView &G, const uint32_t *vbits,
                           const int2 *qlist, const int *qcount, const float *sr, const float *si, float2 *A) {
-        if constexpr (use_cb<MODE>())
+        if constexpr (fwd_pipe<N>())
+            k_plane_fwd_pipe<N, MODE><<<dim3(NG, nb), FwdPipe<N>::NT, FwdPipe<N>::bytes, s>>>(
+                L, G, vbits, qlist, qcount, sr, si, A);
+        else if constexpr (use_cb<MODE>())
             k_plane_fwd_cb<N, MODE><<<dim3(NG, nb), kNT1B, fwd_cb_smem<N>(), s>>>(L, G, vbits, qlist, qcount, sr, si, A);
         else
             k_plane_fwd<N, MODE><<<dim3(NG, nb), kNT1, smem_fwd(), s>>>(L, G, vbits, qlist, qcount, sr, si, A);

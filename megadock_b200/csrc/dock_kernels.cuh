@@ -6,7 +6,7 @@
 //                  plane p (rPSC real part + charge imaginary part, bit-exact
 //                  with MEGADOCK's CPU path), 2D forward FFT over (y, z) in
 //                  shared memory, store the plane's spectrum  A[p][ky][kz].
-//   K2 xline       (rotation, ky, 32 kz lines): forward FFT along x of the
+//   K2 xline       (rotation, ky, 16 or 8 kz lines): forward FFT along x of the
 //                  ng non-zero planes, multiply by conj(R^), inverse FFT along
 //                  x, store G[x][ky][kz].
 //   K3 plane_inv   (rotation, x-plane): inverse FFT over (ky, kz) -> real score
@@ -678,18 +678,150 @@ __global__ void __launch_bounds__(kNT1, 1)
     }
 }
 
-// K1, column-block form (MODE 0): the same forward plane transform with about
-// half the shared memory, so two CTAs share an SM (used by the batched
-// pipeline wherever two fit: N <= 128; B200 measurement at 12,800 rotations
-// and 64 per launch: 6-10 % more rotations/s at N = 64..112, 0.6 % at 128,
-// identical poses).  The z-FFT results of the
-// NG non-zero rows stay resident (NG x (N+1)); the y-FFT then runs over
-// blocks of CB columns through an N x (CB+1) buffer: pruned phase 1 from the
-// resident rows into the block buffer, phase 2 from the block buffer
-// straight to global memory.
-constexpr int kNT1B = 512;
-
+// K1, pipelined form: the z-FFT results of the NG non-zero rows stay resident
+// and the y-FFT runs over blocks of W columns through two block buffers, one
+// half of the CTA in pass 1 of a block (resident rows -> buffer) while the
+// other is in pass 2 of the block before (buffer -> global memory): one barrier
+// per block, an item per thread, and the shared-memory pass overlaps the
+// stores.  Rows keep their R1 blocks at the odd stride STR, so the z pass ends
+// in place (block u, place k2 holds kz = u + R1 k2) without a trip through
+// registers, and lanes over kz read the blocks without bank conflicts.  us per
+// rotation against the column-block form below (B200): N = 48 0.25 -> 0.17, 72
+// 0.64 -> 0.50, 84 0.93 -> 0.91; the whole graph with two launch groups in
+// flight 48 0.79 -> 0.71, 64 1.35 -> 1.29, 72 2.49 -> 2.33, 84 3.86 -> 3.83, 90
+// equal, 96 4.85 -> 5.04 (its CTAs leave the other group less room).  From 108
+// on two CTAs of 340 to 400 threads lose to two of 512 (1.90 -> 2.14, 128 2.32
+// -> 2.70), and as the only CTA of an SM to the one-CTA form (160 6.2 -> 6.6).
 constexpr size_t kSmemMax = 227 * 1024;   // dynamic shared memory one CTA may hold
+
+template <int N>
+struct FwdPipe {
+    static constexpr int R1 = Plan<N>::R1, R2 = Plan<N>::R2, NG = N / 2;
+    static constexpr int STR = R2 | 1, PZ = (R1 * STR) | 1;
+    static constexpr int W = 16;
+    static constexpr int T1 = (W * R2 + 31) / 32 * 32, T2 = (W * R1 + 31) / 32 * 32, NT = T1 + T2;
+    static constexpr size_t bytes = ((size_t)NG * PZ + 2 * (size_t)N * (W + 1)) * sizeof(float2);
+    static constexpr int OCC_S = (int)((227 * 1024) / (bytes + 1024)), OCC_R = 65536 / (NT * 72), OCC_T = 2048 / NT;
+    static constexpr int OCC0 = OCC_S < OCC_R ? OCC_S : OCC_R;
+    static constexpr int OCC = (OCC0 < OCC_T ? OCC0 : OCC_T) > 0 ? (OCC0 < OCC_T ? OCC0 : OCC_T) : 1;
+};
+
+template <int N>
+constexpr bool fwd_pipe() {
+    return N <= 84;
+}
+
+template <int N, int MODE = 0>
+__global__ void __launch_bounds__(FwdPipe<N>::NT, FwdPipe<N>::OCC)
+    k_plane_fwd_pipe(LigandView L, GridView G, const uint32_t *__restrict__ vbits, const int2 *__restrict__ qlist,
+                     const int *__restrict__ qcount, const float *__restrict__ src_r, const float *__restrict__ src_i,
+                     float2 *__restrict__ A) {
+    using P = FwdPipe<N>;
+    constexpr int NG = N / 2, OFF = N / 4, R1 = P::R1, R2 = P::R2, STR = P::STR, PZ = P::PZ, BW = P::W, PY = BW + 1;
+    constexpr int NT = P::NT, W = VoxShared<NG>::W;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    float2 *Z = reinterpret_cast<float2 *>(smem_raw);   // NG rows x PZ
+    float2 *Y = Z + NG * PZ;                             // 2 x N rows x PY
+    const int p = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+    // element of voxel column s in row q
+    auto at = [&](int q, int s) -> float2 & {
+        const int z = s + OFF;
+        return Z[q * PZ + (z / R2) * STR + z % R2];
+    };
+    if constexpr (MODE == 1) {
+        for (int c = tid; c < NG * NG; c += NT) {
+            const int q = c / NG, s = c % NG;
+            const size_t gidx = ((size_t)p * NG + q) * NG + s;
+            at(q, s) = make_float2(src_r[gidx], src_i[gidx]);
+        }
+        __syncthreads();
+    } else {
+        const uint32_t *vb = vbits + ((size_t)b * NG + p) * 2 * NG * W;
+        // the cells of this thread with a compile-time trip count and both
+        // class words loaded unconditionally: the loads of eight are in flight
+        constexpr int CPT = (NG * NG + NT - 1) / NT;
+#pragma unroll 8
+        for (int r = 0; r < CPT; ++r) {
+            const int c = tid + r * NT;
+            if (NG * NG % NT == 0 || c < NG * NG) {
+                const int q = c / NG, s = c % NG;
+                const uint32_t bit = 1u << (s & 31);
+                const uint32_t w2 = __ldg(&vb[q * W + (s >> 5)]), w1 = __ldg(&vb[NG * W + q * W + (s >> 5)]);
+                const float v = (w2 & bit) ? L.delta : (w1 & bit) ? 1.0f : 0.0f;
+                at(q, s) = make_float2(v, 0.f);
+            }
+        }
+        __syncthreads();
+        const int nq = qcount[(size_t)b * NG + p];
+        const int2 *ql = qlist + ((size_t)b * NG + p) * NG * NG;
+        for (int e = tid; e < nq; e += NT) {
+            const int2 c = ql[e];
+            at(c.x / NG, c.x % NG).y = __int_as_float(c.y);
+        }
+        __syncthreads();
+    }
+    // z-FFT of the NG rows (lanes = rows), both passes in place
+    for (int it = tid; it < NG * R2; it += NT) {
+        const int t = it / NG;
+        float2 *row = Z + (it % NG) * PZ + t;
+        float2 v[R1];
+        padded_inputs<N, R1, R2>(v, t, [&](int y) { return row[(y + OFF - t) / R2 * STR]; });
+        Dft<R1, -1>::run(v);
+        static_for<0, R1>([&](auto k1_) {
+            constexpr int k1 = decltype(k1_)::value;
+            float2 x = v[k1];
+            if constexpr (k1 != 0) x = cmul(x, __ldg(&G.tw[t * k1]));
+            row[k1 * STR] = x;
+        });
+    }
+    __syncthreads();
+    for (int it = tid; it < NG * R1; it += NT) {
+        float2 *row = Z + (it % NG) * PZ + (it / NG) * STR;
+        float2 v[R2];
+        static_for<0, R2>([&](auto n2) { v[n2] = row[n2]; });
+        Dft<R2, -1>::run(v);
+        static_for<0, R2>([&](auto k2) { row[k2] = v[k2]; });
+    }
+    __syncthreads();
+    // y-FFT of the N columns
+    float2 *Ab = A + ((size_t)b * NG + p) * N * N;
+    constexpr int NB = (N + BW - 1) / BW;
+    const bool first = tid < P::T1;
+    const int it = first ? tid : tid - P::T1, c = it % BW, k = it / BW;   // k = t (pass 1) or u (pass 2)
+    const bool live = first ? k < R2 : k < R1;
+    for (int blk = 0; blk <= NB; ++blk) {
+        if (first) {
+            const int kz = blk * BW + c;
+            if (live && blk < NB && (N % BW == 0 || kz < N)) {
+                const float2 *col = Z + (kz % R1) * STR + kz / R1;
+                float2 *dst = Y + (blk & 1) * N * PY + k * PY + c;
+                float2 v[R1];
+                padded_inputs<N, R1, R2>(v, k, [&](int q) { return col[q * PZ]; });
+                Dft<R1, -1>::run(v);
+                static_for<0, R1>([&](auto k1_) {
+                    constexpr int k1 = decltype(k1_)::value;
+                    float2 x = v[k1];
+                    if constexpr (k1 != 0) x = cmul(x, __ldg(&G.tw[k * k1]));
+                    dst[k1 * R2 * PY] = x;
+                });
+            }
+        } else {
+            const int kz = (blk - 1) * BW + c;
+            if (live && blk > 0 && (N % BW == 0 || kz < N)) {
+                float2 o[R2];
+                fft_phase2<N, -1>(Y + ((blk - 1) & 1) * N * PY + c, PY, k, o);
+                static_for<0, R2>([&](auto k2) { Ab[(size_t)(k + R1 * k2) * N + kz] = o[k2]; });
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// K1, column-block form (84 < N <= 128, two CTAs per SM, and above 168, where
+// the one-CTA form does not fit): the resident z-transformed rows (NG x (N+1))
+// and one N x (CB+1) block buffer: pruned phase 1 from the resident rows into
+// the buffer, phase 2 from the buffer straight to global memory.
+constexpr int kNT1B = 512;
 
 template <int N>
 constexpr size_t fwd_cb_smem_of(int cb) {
