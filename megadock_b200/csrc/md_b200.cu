@@ -138,6 +138,22 @@ int group_of(const md_ctx *ctx, int n, int t) {
     return std::max(1, (n + groups - 1) / groups);
 }
 
+// The work set and scratch(B) of a call in groups of B rotations; where an
+// automatic group has no room on the device, of one rotation (B becomes 1).
+template <class Scratch>
+int with_group(md_ctx *ctx, int &B, const Scratch &scratch) {
+    int rc = ensure_work(ctx, B, 1);
+    if (!rc) rc = scratch(B);
+    if (rc && ctx->batch == 0 && B > 1) {
+        cudaGetLastError();
+        release_work(ctx);
+        B = 1;
+        rc = ensure_work(ctx, B, 1);
+        if (!rc) rc = scratch(B);
+    }
+    return rc;
+}
+
 int check_ready(md_ctx *ctx) {
     if (!ctx->N) {
         ctx->err = "md_set_grid has not been called";
@@ -157,6 +173,13 @@ int check_ready(md_ctx *ctx) {
 // The rotation loop of one md_dock call on device buffers.
 int run_dock(md_ctx *ctx, const float *d_rot, int first_rot, int n_rot, int t, DevPose *d_pose) {
     int B = group_of(ctx, n_rot, t);
+    if (ctx->batch == 0 && B > ctx->cap) {
+        // a caller capturing its stream gets the work set that is there: no
+        // allocation may fall inside a capture
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(ctx->stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
+            B = std::max(1, ctx->cap);
+    }
     const bool batched = ctx->batch != 0 && B > 1;
     int rc = ensure_work(ctx, B, t, batched ? ctx->lanes : 1);
     if (rc && ctx->batch == 0 && B > 1) {
@@ -694,16 +717,17 @@ int adjoint_core(md_ctx *ctx, const float *rotmat, int n, const int4 *shift, con
     MD_CUDA(cudaSetDevice(ctx->device));
     const int N = ctx->N, ng = ctx->ng;
     const size_t ng3 = (size_t)ng * ng * ng;
-    const int B = group_of(ctx, n, 1);
-    int rc = ensure_work(ctx, B, 1);
-    if (rc) return rc;
-    const size_t sz[9] = {sizeof(float) * 9 * n,       sizeof(float) * n,
-                          sizeof(int4) * n,            sizeof(float) * 2 * ng3,
-                          sizeof(float) * 2 * ng3 * B, sizeof(float) * std::max(ctx->na, 1),
-                          sizeof(int) * std::max(n_lig, 1), sizeof(float) * 2 * ng3 * std::max(n_lig, 0),
-                          sizeof(double) * kAdjBlocks};
+    int B = group_of(ctx, n, 1);
     char *p[9];
-    if ((rc = carve_scratch(ctx, sz, 9, p))) return rc;
+    int rc = with_group(ctx, B, [&](int b) {
+        const size_t sz[9] = {sizeof(float) * 9 * n,       sizeof(float) * n,
+                              sizeof(int4) * n,            sizeof(float) * 2 * ng3,
+                              sizeof(float) * 2 * ng3 * b, sizeof(float) * std::max(ctx->na, 1),
+                              sizeof(int) * std::max(n_lig, 1), sizeof(float) * 2 * ng3 * std::max(n_lig, 0),
+                              sizeof(double) * kAdjBlocks};
+        return carve_scratch(ctx, sz, 9, p);
+    });
+    if (rc) return rc;
     float *d_rot = reinterpret_cast<float *>(p[0]), *d_w = reinterpret_cast<float *>(p[1]);
     int4 *d_shift = reinterpret_cast<int4 *>(p[2]);
     float *d_grad = reinterpret_cast<float *>(p[3]), *d_vox = reinterpret_cast<float *>(p[4]);
@@ -872,11 +896,13 @@ int md_pose_scores(md_ctx *ctx, const float *rotmat, int n, const md_pose *poses
         }
         shift[r] = make_int4(poses[r].i, poses[r].j, poses[r].k, 0);
     }
-    const int B = group_of(ctx, n, 1);
-    if ((rc = ensure_work(ctx, B, 1))) return rc;
-    const size_t sz[4] = {sizeof(float) * 9 * n, sizeof(int4) * n, sizeof(float) * n, sizeof(float) * 2 * ng3 * B};
+    int B = group_of(ctx, n, 1);
     char *p[4];
-    if ((rc = carve_scratch(ctx, sz, 4, p))) return rc;
+    rc = with_group(ctx, B, [&](int b) {
+        const size_t sz[4] = {sizeof(float) * 9 * n, sizeof(int4) * n, sizeof(float) * n, sizeof(float) * 2 * ng3 * b};
+        return carve_scratch(ctx, sz, 4, p);
+    });
+    if (rc) return rc;
     float *d_rot = reinterpret_cast<float *>(p[0]), *d_sc = reinterpret_cast<float *>(p[2]);
     int4 *d_shift = reinterpret_cast<int4 *>(p[1]);
     float *d_vox = reinterpret_cast<float *>(p[3]);
@@ -923,8 +949,8 @@ int md_pose_terms(md_ctx *ctx, const float *rec_rpsc, const float *rotmat, int n
     const size_t ng3 = (size_t)ng * ng * ng;
     // poses per launch: their voxel grids within about 1 GB
     const int P = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, ((size_t)1 << 30) / (8 * ng3)));
-    const int B = group_of(ctx, P, 1);
-    if ((rc = ensure_work(ctx, B, 1))) return rc;
+    int B = group_of(ctx, P, 1);
+    if ((rc = with_group(ctx, B, [](int) { return MD_OK; }))) return rc;
     float *d_rot = nullptr, *d_vox = nullptr, *d_terms = nullptr, *d_rpsc = nullptr;
     int4 *d_tem = nullptr;
     cudaError_t e = cudaSuccess;
