@@ -92,7 +92,8 @@ class FFTProcess:
         _check(N.lib().md_release_work(self._h), self._h)
 
     def set_tile(self, lines: int):
-        """kz lines per CTA of the x-line kernel (8, 16 or 32)."""
+        """Tile width asked of the x-line kernel (8, 16 or 32; every size has one
+        shape, so it selects nothing)."""
         _check(N.lib().md_set_tile(self._h, int(lines)), self._h)
         self.tile = int(lines)
 
@@ -102,7 +103,8 @@ class FFTProcess:
         self.lanes = int(lanes)
 
     def set_plan(self, plan: int):
-        """Radix plan variant of the inverse plane kernel (0, 1 or 2)."""
+        """Radix plan variant of the inverse plane kernel (0, 1 or 2; they differ
+        at N = 128)."""
         _check(N.lib().md_set_plan(self._h, int(plan)), self._h)
         self.plan = int(plan)
 

@@ -2,14 +2,13 @@
 
 The batched pipeline's cost per rotation falls as more rotations share a
 launch (fuller grids, fewer launches) until the per-launch intermediates stop
-fitting in L2, and the inverse plane kernel (the largest stage) runs at
-different speeds with different radix splits of its two axes (md_set_plan:
-variant 0 the line plans, 1 the kz split reversed, 2 the ky split reversed),
-depending on the size, and the x-line kernel works on tiles of 8, 16 or 32
-kz lines per CTA (md_set_tile).  ``autotune`` times a sample of rotations with
-the library's per-stage CUDA events (md_dock_profile): first every batch size
-with plan 0 and 32-line tiles, then every plan at the best batch, then the
-other tiles, and keeps the fastest combination.  Last it times the whole
+fitting in L2; at N = 128 the inverse plane kernel has two radix plans
+(md_set_plan), at every other size one measured plan; the x-line kernel has one
+tile shape per size (md_set_tile selects nothing any more, its candidates time
+the same).  ``autotune`` times a sample of rotations with the library's
+per-stage CUDA events (md_dock_profile): first every batch size with plan 0,
+then every plan and tile at the best batch, and keeps the fastest.  Last it
+times the whole
 batched graph (md_dock_device) with one and with two launch groups in flight
 (md_set_lanes): the per-stage events serialise the stages, so they cannot see
 how two groups' kernels share the GPU.  Batch sizes whose two work
