@@ -76,11 +76,16 @@ int md_ligand_data(md_ctx *ctx, int na, const float *xyz_centred, const float *r
 /* Rotations per launch for md_dock (1 = the plain per-rotation pipeline;
  * > 1 = the batched form, launched as one captured CUDA graph).  A context
  * that never gets a value launches groups of rotations that fit a work set of
- * 1 GiB (one rotation where even that has no room), without a graph. */
+ * 1 GiB (one rotation where even that has no room), without a graph.  On a
+ * stream that the caller is capturing such a call takes groups of the size the
+ * context already holds buffers for (one rotation when nothing was docked yet). */
 int md_set_batch(md_ctx *ctx, int rotations_per_launch);
 /* Free the context's rotation work buffers and captured graphs (receptor,
  * ligand and settings stay); the next docking call allocates them again for
- * its launch shape.  The autotuner calls it after trying large launch groups. */
+ * its launch shape.  The autotuner calls it after trying large launch groups.
+ * Buffers that a caller's own stream capture recorded stay until this call,
+ * another FFT edge or the end of the context, also when later calls need larger
+ * ones; a graph of the caller's must not be replayed after any of the three. */
 int md_release_work(md_ctx *ctx);
 /* Radix plan of the inverse plane kernel (0, 1 or 2; other values are
  * refused).  At FFT edge 128 it picks the line plans, the kz split reversed or

@@ -121,6 +121,11 @@ struct md_ctx {
     WorkSet::Sizes have{};           // bytes held by each work-set buffer
     int sets = 0;                    // work sets allocated (1 or kLanes)
     WorkSet ws[kLanes];
+    // A caller that captures its stream records the work sets' addresses: from
+    // then on they are replaced by larger ones but not freed (`kept`) until
+    // md_release_work, another grid edge or the context's end.
+    bool lent = false;
+    std::vector<WorkSet> kept;
     char *d_scratch = nullptr;   // scratch of the adjoint and pose-scoring calls (grows to the largest call)
     size_t scratch_cap = 0;
     // staging for host-buffer calls

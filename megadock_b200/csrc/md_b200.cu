@@ -54,20 +54,48 @@ void free_graphs(md_ctx *c) {
     c->pair_graphs.clear();
 }
 
-void release_work(md_ctx *c) {
-    free_graphs(c);
-    for (auto &w : c->ws) w.release();
+void free_scratch(md_ctx *c) {
     cudaFree(c->d_scratch);
     c->d_scratch = nullptr;
     c->scratch_cap = 0;
+}
+
+// The work sets go (free), or move to `kept` where a caller's graph holds them.
+void drop_sets(md_ctx *c) {
+    free_graphs(c);
+    for (auto &w : c->ws) {
+        if (c->lent && w.A) {
+            c->kept.push_back(w);
+            w = WorkSet();
+        } else {
+            w.release();
+        }
+    }
+    c->lent = false;
     c->cap = c->cap_t = c->cap_na = 0;
     c->sets = 0;
     c->have = WorkSet::Sizes{};
 }
 
+void release_work(md_ctx *c) {
+    drop_sets(c);
+    for (auto &w : c->kept) w.release();
+    c->kept.clear();
+    free_scratch(c);
+}
+
+// Notes that the stream's capture, if the caller has one open, records the
+// addresses of the work sets.
+void lend_to_capture(md_ctx *c) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) c->lent = true;
+}
+
 // At least `nsets` work sets holding at least `z` bytes per buffer (only the
 // batched graph with two launch groups in flight and the pairs runner use the
 // second set, so one launch group in flight holds one set on the device).
+// Where the device has no room for them, sets that a caller's graph holds stay
+// as they are; others are gone already, so that the new ones can take their place.
 int ensure_bytes(md_ctx *ctx, const WorkSet::Sizes &z, int nsets) {
     bool ok = ctx->sets >= nsets;
     for (int k = 0; k < WorkSet::kBufs; ++k) ok = ok && z.b[k] <= ctx->have.b[k];
@@ -75,8 +103,19 @@ int ensure_bytes(md_ctx *ctx, const WorkSet::Sizes &z, int nsets) {
     WorkSet::Sizes m = ctx->have;
     for (int k = 0; k < WorkSet::kBufs; ++k) m.b[k] = std::max(m.b[k], z.b[k]);
     const int cap = ctx->cap, t = ctx->cap_t, na = ctx->cap_na;
-    release_work(ctx);
-    for (int k = 0; k < nsets; ++k) MD_CUDA(ctx->ws[k].allocate(m));
+    free_scratch(ctx);
+    if (!ctx->lent) drop_sets(ctx);
+    WorkSet fresh[kLanes];
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < nsets && e == cudaSuccess; ++k) e = fresh[k].allocate(m);
+    if (e != cudaSuccess) {
+        for (auto &w : fresh) w.release();
+        cudaGetLastError();
+        ctx->err = std::string("work buffers: ") + cudaGetErrorString(e);
+        return MD_ERR_CUDA;
+    }
+    if (ctx->lent) drop_sets(ctx);
+    for (int k = 0; k < nsets; ++k) ctx->ws[k] = fresh[k];
     ctx->sets = nsets;
     ctx->have = m;
     ctx->cap = cap;
@@ -111,9 +150,7 @@ int carve_scratch(md_ctx *ctx, const size_t *sz, int n, char **out) {
     }
     if (total > ctx->scratch_cap) {
         MD_CUDA(cudaStreamSynchronize(ctx->stream));
-        cudaFree(ctx->d_scratch);
-        ctx->d_scratch = nullptr;
-        ctx->scratch_cap = 0;
+        free_scratch(ctx);
         MD_CUDA(cudaMalloc(&ctx->d_scratch, total));
         ctx->scratch_cap = total;
     }
@@ -146,7 +183,8 @@ int with_group(md_ctx *ctx, int &B, const Scratch &scratch) {
     if (!rc) rc = scratch(B);
     if (rc && ctx->batch == 0 && B > 1) {
         cudaGetLastError();
-        release_work(ctx);
+        free_scratch(ctx);
+        if (!ctx->lent) drop_sets(ctx);
         B = 1;
         rc = ensure_work(ctx, B, 1);
         if (!rc) rc = scratch(B);
@@ -189,6 +227,7 @@ int run_dock(md_ctx *ctx, const float *d_rot, int first_rot, int n_rot, int t, D
         rc = ensure_work(ctx, B, t);
     }
     if (rc) return rc;
+    lend_to_capture(ctx);
     if (!batched) {
         // plain form (one rotation per fused pipeline) and automatic groups,
         // launched back to back
@@ -663,6 +702,7 @@ int md_dock_pairs(md_ctx *runner, md_ctx *const *pairs, int npairs, const float 
     }
     int rc = ensure_bytes(ctx, z, kLanes);
     if (rc) return rc;
+    lend_to_capture(ctx);
     auto it = ctx->pair_graphs.find(key);
     if (it == ctx->pair_graphs.end()) {
         // keys of changed or destroyed pair contexts never match again: bound the cache

@@ -1,0 +1,150 @@
+"""Work buffers of a context on the CPU: the library's host side linked against
+a CUDA runtime without a device (tests/fake_runtime), whose device memory is a
+ledger under a budget.  Covers what no run on a GPU shows without a fault or an
+exhausted device: which buffers a captured launch keeps using, what a context
+does where its automatic launch groups have no room."""
+import ctypes as C
+import shutil
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+CSRC = ROOT / "megadock_b200" / "csrc"
+FAKE = ROOT / "tests" / "fake_runtime"
+NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+MIB = 1 << 20
+
+
+@pytest.fixture(scope="module")
+def rt(tmp_path_factory):
+    """md_b200.cu and the fake runtime as one library (device code as PTX only)."""
+    if not Path(NVCC).exists():
+        pytest.skip("no nvcc")
+    d = tmp_path_factory.mktemp("fake")
+    flags = [NVCC, "-std=c++17", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=compute_100a",
+             "-Xcompiler", "-fPIC", "-c"]
+    jobs = [subprocess.Popen(flags + ["-o", str(d / f"{src.stem}.o"), str(src)], stderr=subprocess.PIPE, text=True)
+            for src in (CSRC / "md_b200.cu", FAKE / "fake_sizes.cu", FAKE / "fake_runtime.cpp")]
+    for j in jobs:
+        _, err = j.communicate()
+        assert j.returncode == 0, err
+    so = d / "libfake.so"
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", str(so), *map(str, d.glob("*.o"))], check=True)
+    lib = C.CDLL(str(so))
+    from megadock_b200._native import _PROTOS
+    for name, (res, args) in _PROTOS.items():
+        if hasattr(lib, name):
+            getattr(lib, name).restype, getattr(lib, name).argtypes = res, args
+    lib.fake_used.restype = C.c_size_t
+    lib.fake_budget.argtypes = [C.c_size_t]
+    return lib
+
+
+class Context:
+    """A context with a grid, a receptor and a ligand of 20 atoms."""
+
+    def __init__(self, rt, n, batch=0, device=0):
+        self.rt, self.n = rt, n
+        self.h = C.c_void_p()
+        assert rt.md_ctx_create(device, C.byref(self.h)) == 0
+        ng = n // 2
+        z = np.zeros(ng ** 3)
+        self.ok(rt.md_set_grid(self.h, n, 1.2, _f(np.arange(ng))))
+        if batch:
+            self.ok(rt.md_set_batch(self.h, batch))
+        self.ok(rt.md_receptor_fft(self.h, _f(z), _f(z)))
+        a = np.ones(60)
+        self.ok(rt.md_ligand_data(self.h, 20, _f(a), _f(a), _f(a), 1.0))
+
+    def ok(self, rc):
+        assert rc == 0, self.rt.md_last_error(self.h).decode()
+
+    def dock(self, n, t=1):
+        out = np.zeros(5 * n * t, np.int32)
+        self.ok(self.rt.md_dock(self.h, _f(np.zeros(9 * n)), 0, n, t, out.ctypes.data))
+
+    def dock_device(self, n, t=1):
+        self.ok(self.rt.md_dock_device(self.h, C.c_void_p(1 << 20), 0, n, t, C.c_void_p(1 << 21)))
+
+    def pose_scores(self, n):
+        poses = np.zeros(5 * n, np.int32)
+        self.ok(self.rt.md_pose_scores(self.h, _f(np.zeros(9 * n)), n, poses.ctypes.data, _f(np.zeros(n))))
+
+    def capture(self, n, t=1):
+        """The launches of md_dock_device on a stream the caller is capturing."""
+        first = self.rt.fake_launches()
+        self.rt.fake_capture(1)
+        self.dock_device(n, t)
+        self.rt.fake_capture(0)
+        return range(first, self.rt.fake_launches())
+
+    def close(self):
+        self.rt.md_ctx_destroy(self.h)
+
+
+def _f(a):
+    return np.ascontiguousarray(a, np.float32).ctypes.data_as(C.POINTER(C.c_float))
+
+
+@pytest.fixture
+def context(rt):
+    made = []
+
+    def make(*a, **k):
+        made.append(Context(rt, *a, **k))
+        return made[-1]
+
+    rt.fake_budget(1 << 62)
+    yield make
+    rt.fake_capture(0)
+    for c in made:
+        c.close()
+    rt.fake_forget()
+    assert rt.fake_used() == 0
+    assert rt.fake_short() == 0   # no launch got freed or too small buffers
+
+
+@pytest.mark.parametrize("batch", [0, 1])
+@pytest.mark.parametrize("n", [48, 128, 256])
+def test_captured_launches_keep_their_buffers(rt, context, n, batch):
+    """What a caller captured stays valid through later calls that need larger
+    buffers (more rotations, poses per rotation, rotations per launch), and
+    until the caller gives the work buffers back."""
+    c = context(n, batch)
+    c.dock(2)
+    held = list(c.capture(5))
+    larger = [lambda: c.dock(200), lambda: c.dock(3, t=40), lambda: c.pose_scores(64)]
+    for call in larger:
+        call()
+        held += c.capture(4)
+    c.ok(rt.md_set_batch(c.h, 300))
+    c.dock(300)
+    assert len(held) > 4 and all(rt.fake_live(k) for k in held)
+    c.ok(rt.md_release_work(c.h))
+    assert not any(rt.fake_live(k) for k in held)
+    c.dock(2)
+
+
+def test_captured_launches_survive_a_failed_growth(rt, context):
+    c = context(48)
+    c.dock(2)
+    held = c.capture(2)
+    rt.fake_budget(rt.fake_used() + 1 * MIB)
+    c.dock(100)
+    c.pose_scores(20)
+    assert all(rt.fake_live(k) for k in held)
+
+
+def test_uncaptured_work_buffers_do_not_add_up(rt, context):
+    """Without a capture a growing call replaces the buffers."""
+    a, b = context(48), context(48)
+    before = rt.fake_used()
+    for n in (1, 2, 7, 40, 64):
+        a.dock(n)
+    grown = rt.fake_used() - before
+    before = rt.fake_used()
+    b.dock(64)
+    assert grown == rt.fake_used() - before
