@@ -25,7 +25,7 @@ def rt(tmp_path_factory):
         pytest.skip("no nvcc")
     d = tmp_path_factory.mktemp("fake")
     flags = [NVCC, "-std=c++17", "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=compute_100a",
-             "-Xcompiler", "-fPIC", "-c"]
+             "-Xcompiler", "-fPIC,-fno-gnu-unique", "-c"]   # nothing shared with the real library
     jobs = [subprocess.Popen(flags + ["-o", str(d / f"{src.stem}.o"), str(src)], stderr=subprocess.PIPE, text=True)
             for src in (CSRC / "md_b200.cu", FAKE / "fake_sizes.cu", FAKE / "fake_runtime.cpp")]
     for j in jobs:
