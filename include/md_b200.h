@@ -76,7 +76,8 @@ int md_ligand_data(md_ctx *ctx, int na, const float *xyz_centred, const float *r
 /* Rotations per launch for md_dock (1 = the plain per-rotation pipeline;
  * > 1 = the batched form, launched as one captured CUDA graph).  A context
  * that never gets a value launches groups of rotations that fit a work set of
- * 1 GiB (one rotation where even that has no room), without a graph.  On a
+ * 1 GiB, without a graph (one rotation where even that has no room, from then on
+ * until md_release_work).  On a
  * stream that the caller is capturing such a call takes groups of the size the
  * context already holds buffers for (one rotation when nothing was docked yet). */
 int md_set_batch(md_ctx *ctx, int rotations_per_launch);

@@ -80,6 +80,7 @@ struct WorkSet {
 };
 
 constexpr int kLanes = 2;
+constexpr int kAutoGroup = 64;   // rotations per launch, at most, where the context chooses (group_of)
 
 }  // namespace
 
@@ -114,6 +115,7 @@ struct md_ctx {
     bool have_ligand = false;
     // work sets (lane 0 serves every form; lane 1 the batched graph)
     int batch = 0;   // rotations per launch asked for (md_set_batch); 0 = never asked (group_of)
+    int auto_most = kAutoGroup;   // 1 once larger automatic groups had no room (reserve_groups)
     int plan = 0;   // radix plan variant of the plane top-t kernel (C2RPlan)
     int tile = 32;  // md_set_tile's value: every size has one x-line shape (XPlan), so it selects nothing
     int lanes = kLanes;   // work sets / capture streams the batched graph alternates over (1 or 2)

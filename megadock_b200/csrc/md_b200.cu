@@ -82,13 +82,13 @@ void release_work(md_ctx *c) {
     for (auto &w : c->kept) w.release();
     c->kept.clear();
     free_scratch(c);
+    c->auto_most = kAutoGroup;
 }
 
-// Notes that the stream's capture, if the caller has one open, records the
-// addresses of the work sets.
-void lend_to_capture(md_ctx *c) {
+// Whether the caller is capturing the context's stream.
+bool capture_open(const md_ctx *c) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) c->lent = true;
+    return cudaStreamIsCapturing(c->stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone;
 }
 
 // At least `nsets` work sets holding at least `z` bytes per buffer (only the
@@ -160,36 +160,47 @@ int carve_scratch(md_ctx *ctx, const size_t *sz, int n, char **out) {
 
 // Rotations per launch of a call over n: md_set_batch's value, or, in a context
 // that never got one, as many as keep the work set within kAutoBytes, at most
-// kAutoGroup, in groups of even size.  One rotation leaves most of the GPU
-// idle (64 to 2,000 CTAs a kernel at N = 128) and pays nine launches: B200,
+// `auto_most`, in groups of even size.  One rotation leaves most of the GPU
+// idle (64 to 2,000 CTAs a kernel at N = 128) and pays seven launches: B200,
 // 360 rotations at N = 128, t = 3, from host buffers: 30.5 -> 4.3 ms.
 constexpr size_t kAutoBytes = size_t(1) << 30;
-constexpr int kAutoGroup = 64;
-int group_of(const md_ctx *ctx, int n, int t) {
+int group_of(const md_ctx *ctx, int n, int t, int auto_most) {
     if (ctx->batch) return std::max(1, std::min(ctx->batch, n));
     const WorkSet::Sizes z = WorkSet::need(1, ctx->N, t, std::max(ctx->na, 1));
     size_t one = 0;
     for (size_t b : z.b) one += b;
-    const int most = (int)std::max<size_t>(1, std::min<size_t>(kAutoGroup, kAutoBytes / one));
+    const int most = (int)std::max<size_t>(1, std::min<size_t>(auto_most, kAutoBytes / one));
     const int groups = (std::max(n, 1) + most - 1) / most;
     return std::max(1, (n + groups - 1) / groups);
 }
 
-// The work set and scratch(B) of a call in groups of B rotations; where an
-// automatic group has no room on the device, of one rotation (B becomes 1).
-template <class Scratch>
-int with_group(md_ctx *ctx, int &B, const Scratch &scratch) {
-    int rc = ensure_work(ctx, B, 1);
-    if (!rc) rc = scratch(B);
-    if (rc && ctx->batch == 0 && B > 1) {
+// Runs `reserve`, which picks a call's group sizes and allocates for them.  Where
+// automatic groups have no room on the device it runs again with groups of one
+// rotation, and the context keeps to those until its work buffers are released,
+// so that later calls do not repeat the attempt.
+template <class Reserve>
+int reserve_groups(md_ctx *ctx, bool automatic, const Reserve &reserve) {
+    int rc = reserve();
+    if (rc == MD_ERR_CUDA && automatic && ctx->auto_most > 1) {
         cudaGetLastError();
         free_scratch(ctx);
         if (!ctx->lent) drop_sets(ctx);
-        B = 1;
-        rc = ensure_work(ctx, B, 1);
-        if (!rc) rc = scratch(B);
+        ctx->auto_most = 1;
+        rc = reserve();
+        if (rc) ctx->auto_most = kAutoGroup;
     }
+    if (rc) cudaGetLastError();   // a refused allocation is reported once, here
     return rc;
+}
+
+// The work set and scratch(B) of a call over n in groups of B rotations.
+template <class Scratch>
+int with_group(md_ctx *ctx, int n, int &B, const Scratch &scratch) {
+    return reserve_groups(ctx, ctx->batch == 0, [&]() {
+        B = group_of(ctx, n, 1, ctx->auto_most);
+        const int rc = ensure_work(ctx, B, 1);
+        return rc ? rc : scratch(B);
+    });
 }
 
 int check_ready(md_ctx *ctx) {
@@ -210,24 +221,19 @@ int check_ready(md_ctx *ctx) {
 
 // The rotation loop of one md_dock call on device buffers.
 int run_dock(md_ctx *ctx, const float *d_rot, int first_rot, int n_rot, int t, DevPose *d_pose) {
-    int B = group_of(ctx, n_rot, t);
-    if (ctx->batch == 0 && B > ctx->cap) {
+    int B = 1;
+    bool batched = false;
+    const bool capturing = capture_open(ctx);
+    const int rc = reserve_groups(ctx, ctx->batch == 0 && !capturing, [&]() {
+        B = group_of(ctx, n_rot, t, ctx->auto_most);
         // a caller capturing its stream gets the work set that is there: no
         // allocation may fall inside a capture
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(ctx->stream, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone)
-            B = std::max(1, ctx->cap);
-    }
-    const bool batched = ctx->batch != 0 && B > 1;
-    int rc = ensure_work(ctx, B, t, batched ? ctx->lanes : 1);
-    if (rc && ctx->batch == 0 && B > 1) {
-        // no room for the automatic group: one rotation at a time
-        cudaGetLastError();
-        B = 1;
-        rc = ensure_work(ctx, B, t);
-    }
+        if (ctx->batch == 0 && capturing) B = std::min(B, std::max(1, ctx->cap));
+        batched = ctx->batch != 0 && B > 1;
+        return ensure_work(ctx, B, t, batched ? ctx->lanes : 1);
+    });
     if (rc) return rc;
-    lend_to_capture(ctx);
+    if (capturing) ctx->lent = true;
     if (!batched) {
         // plain form (one rotation per fused pipeline) and automatic groups,
         // launched back to back
@@ -642,8 +648,12 @@ int md_dock_profile(md_ctx *ctx, const float *d_rot, int first_rot, int n_rot, i
     int rc = check_ready(ctx);
     if (rc) return rc;
     MD_CUDA(cudaSetDevice(ctx->device));
-    const int B = group_of(ctx, n_rot, t);
-    if ((rc = ensure_work(ctx, B, t))) return rc;
+    int B = 1;
+    rc = reserve_groups(ctx, ctx->batch == 0, [&]() {
+        B = group_of(ctx, n_rot, t, ctx->auto_most);
+        return ensure_work(ctx, B, t);
+    });
+    if (rc) return rc;
     cudaEvent_t ev[6];
     for (auto &e : ev) MD_CUDA(cudaEventCreate(&e));
     double acc[5] = {0, 0, 0, 0, 0};
@@ -676,9 +686,7 @@ int md_dock_pairs(md_ctx *runner, md_ctx *const *pairs, int npairs, const float 
     md_ctx *ctx = runner;
     if (!ctx || !pairs || !d_rotmat || !n_rot || !d_out || npairs < 0 || t < 1) return MD_ERR_ARG;
     MD_CUDA(cudaSetDevice(ctx->device));
-    // shared work sets: the largest launch group of any pair
-    WorkSet::Sizes z{};
-    std::vector<uintptr_t> key{(uintptr_t)npairs, (uintptr_t)t};
+    bool automatic = false;   // a pair whose groups are chosen here
     for (int p = 0; p < npairs; ++p) {
         md_ctx *c = pairs[p];
         if (!c || !d_rotmat[p] || !d_out[p] || n_rot[p] < 0) return MD_ERR_ARG;
@@ -692,17 +700,29 @@ int md_dock_pairs(md_ctx *runner, md_ctx *const *pairs, int npairs, const float 
             return rc;
         }
         MD_CUDA(set_attrs(c->N));
-        const int B = group_of(c, n_rot[p], t);
-        const WorkSet::Sizes zp = WorkSet::need(B, c->N, t, std::max(c->na, 1));
-        for (int k = 0; k < WorkSet::kBufs; ++k) z.b[k] = std::max(z.b[k], zp.b[k]);
-        // the pair's (uid, gen) stands for every argument the capture takes
-        // from it: grid width, core value, atom count, plan, tile and buffers
-        key.insert(key.end(), {(uintptr_t)c->uid, (uintptr_t)c->gen, (uintptr_t)d_rotmat[p], (uintptr_t)n_rot[p],
-                               (uintptr_t)d_out[p], (uintptr_t)B, (uintptr_t)c->na, (uintptr_t)c->N});
+        automatic = automatic || c->batch == 0;
     }
-    int rc = ensure_bytes(ctx, z, kLanes);
+    // shared work sets: the largest launch group of any pair
+    std::vector<int> group_size(npairs);
+    std::vector<uintptr_t> key;
+    const bool capturing = capture_open(ctx);
+    int rc = reserve_groups(ctx, automatic && !capturing, [&]() {
+        WorkSet::Sizes z{};
+        key = {(uintptr_t)npairs, (uintptr_t)t};
+        for (int p = 0; p < npairs; ++p) {
+            const md_ctx *c = pairs[p];
+            const int B = group_size[p] = group_of(c, n_rot[p], t, ctx->auto_most);
+            const WorkSet::Sizes zp = WorkSet::need(B, c->N, t, std::max(c->na, 1));
+            for (int k = 0; k < WorkSet::kBufs; ++k) z.b[k] = std::max(z.b[k], zp.b[k]);
+            // the pair's (uid, gen) stands for every argument the capture takes
+            // from it: grid width, core value, atom count, plan, tile and buffers
+            key.insert(key.end(), {(uintptr_t)c->uid, (uintptr_t)c->gen, (uintptr_t)d_rotmat[p], (uintptr_t)n_rot[p],
+                                   (uintptr_t)d_out[p], (uintptr_t)B, (uintptr_t)c->na, (uintptr_t)c->N});
+        }
+        return ensure_bytes(ctx, z, kLanes);
+    });
     if (rc) return rc;
-    lend_to_capture(ctx);
+    if (capturing) ctx->lent = true;
     auto it = ctx->pair_graphs.find(key);
     if (it == ctx->pair_graphs.end()) {
         // keys of changed or destroyed pair contexts never match again: bound the cache
@@ -718,7 +738,7 @@ int md_dock_pairs(md_ctx *runner, md_ctx *const *pairs, int npairs, const float 
         int group = 0;
         for (int p = 0; p < npairs; ++p) {
             md_ctx *c = pairs[p];
-            const int B = group_of(c, n_rot[p], t);
+            const int B = group_size[p];
             DevPose *out = reinterpret_cast<DevPose *>(d_out[p]);
             for (int r = 0; r < n_rot[p]; r += B, ++group) {
                 const int nb = std::min(B, n_rot[p] - r);
@@ -757,9 +777,9 @@ int adjoint_core(md_ctx *ctx, const float *rotmat, int n, const int4 *shift, con
     MD_CUDA(cudaSetDevice(ctx->device));
     const int N = ctx->N, ng = ctx->ng;
     const size_t ng3 = (size_t)ng * ng * ng;
-    int B = group_of(ctx, n, 1);
+    int B = 1;
     char *p[9];
-    int rc = with_group(ctx, B, [&](int b) {
+    int rc = with_group(ctx, n, B, [&](int b) {
         const size_t sz[9] = {sizeof(float) * 9 * n,       sizeof(float) * n,
                               sizeof(int4) * n,            sizeof(float) * 2 * ng3,
                               sizeof(float) * 2 * ng3 * b, sizeof(float) * std::max(ctx->na, 1),
@@ -936,9 +956,9 @@ int md_pose_scores(md_ctx *ctx, const float *rotmat, int n, const md_pose *poses
         }
         shift[r] = make_int4(poses[r].i, poses[r].j, poses[r].k, 0);
     }
-    int B = group_of(ctx, n, 1);
+    int B = 1;
     char *p[4];
-    rc = with_group(ctx, B, [&](int b) {
+    rc = with_group(ctx, n, B, [&](int b) {
         const size_t sz[4] = {sizeof(float) * 9 * n, sizeof(int4) * n, sizeof(float) * n, sizeof(float) * 2 * ng3 * b};
         return carve_scratch(ctx, sz, 4, p);
     });
@@ -989,21 +1009,37 @@ int md_pose_terms(md_ctx *ctx, const float *rec_rpsc, const float *rotmat, int n
     const size_t ng3 = (size_t)ng * ng * ng;
     // poses per launch: their voxel grids within about 1 GB
     const int P = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, ((size_t)1 << 30) / (8 * ng3)));
-    int B = group_of(ctx, P, 1);
-    if ((rc = with_group(ctx, B, [](int) { return MD_OK; }))) return rc;
     float *d_rot = nullptr, *d_vox = nullptr, *d_terms = nullptr, *d_rpsc = nullptr;
     int4 *d_tem = nullptr;
+    auto give_back = [&]() {
+        cudaFree(d_rot);
+        cudaFree(d_tem);
+        cudaFree(d_terms);
+        cudaFree(d_rpsc);
+        cudaFree(d_vox);
+        d_rot = d_vox = d_terms = d_rpsc = nullptr;
+        d_tem = nullptr;
+    };
     cudaError_t e = cudaSuccess;
     auto step = [&](cudaError_t x) {
         if (e == cudaSuccess) e = x;
     };
+    int B = 1;
+    rc = with_group(ctx, P, B, [&](int) {
+        e = cudaSuccess;
+        step(cudaMalloc(&d_rot, sizeof(float) * 9 * n));
+        step(cudaMalloc(&d_tem, sizeof(int4) * n));
+        step(cudaMalloc(&d_terms, sizeof(float) * 9 * n));
+        step(cudaMalloc(&d_rpsc, sizeof(float) * ng3));
+        step(cudaMalloc(&d_vox, sizeof(float) * 2 * ng3 * P));
+        if (e == cudaSuccess) return MD_OK;
+        give_back();
+        ctx->err = std::string("pose terms: ") + cudaGetErrorString(e);
+        return MD_ERR_CUDA;
+    });
+    if (rc) return rc;
     std::vector<int4> tem(n);
     for (int p = 0; p < n; ++p) tem[p] = make_int4(tem3[3 * p], tem3[3 * p + 1], tem3[3 * p + 2], 0);
-    step(cudaMalloc(&d_rot, sizeof(float) * 9 * n));
-    step(cudaMalloc(&d_tem, sizeof(int4) * n));
-    step(cudaMalloc(&d_terms, sizeof(float) * 9 * n));
-    step(cudaMalloc(&d_rpsc, sizeof(float) * ng3));
-    step(cudaMalloc(&d_vox, sizeof(float) * 2 * ng3 * P));
     cudaStream_t s = ctx->stream;
     step(cudaMemcpyAsync(d_rot, rotmat, sizeof(float) * 9 * n, cudaMemcpyHostToDevice, s));
     step(cudaMemcpyAsync(d_tem, tem.data(), sizeof(int4) * n, cudaMemcpyHostToDevice, s));
@@ -1025,11 +1061,7 @@ int md_pose_terms(md_ctx *ctx, const float *rec_rpsc, const float *rotmat, int n
         step(cudaMemcpyAsync(terms, d_terms, sizeof(float) * 9 * n, cudaMemcpyDeviceToHost, s));
         step(cudaStreamSynchronize(s));
     }
-    cudaFree(d_rot);
-    cudaFree(d_tem);
-    cudaFree(d_terms);
-    cudaFree(d_rpsc);
-    cudaFree(d_vox);
+    give_back();
     if (e != cudaSuccess) {
         ctx->err = std::string("pose terms: ") + cudaGetErrorString(e);
         return MD_ERR_CUDA;

@@ -17,6 +17,7 @@ uintptr_t next_addr = uintptr_t(1) << 40;
 size_t budget = ~size_t(0), used = 0;
 int refused = 0, device = 0, graphs = 0;
 bool caller_capturing = false;
+cudaError_t last_error = cudaSuccess;
 std::map<int, std::set<const void *>> attrs;   // device -> kernels given their attributes
 
 }  // namespace
@@ -38,7 +39,7 @@ size_t fake_block(uintptr_t addr) {
 cudaError_t cudaMalloc(void **p, size_t n) {
     if (used + n > budget) {
         ++refused;
-        return cudaErrorMemoryAllocation;
+        return last_error = cudaErrorMemoryAllocation;
     }
     *p = reinterpret_cast<void *>(next_addr);
     blocks[next_addr] = n;
@@ -76,7 +77,11 @@ cudaError_t cudaGetDevice(int *d) {
     *d = device;
     return cudaSuccess;
 }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = last_error;
+    last_error = cudaSuccess;
+    return e;
+}
 const char *cudaGetErrorString(cudaError_t e) {
     return e == cudaErrorMemoryAllocation ? "out of memory" : e == cudaSuccess ? "no error" : "error";
 }

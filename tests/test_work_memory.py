@@ -73,6 +73,27 @@ class Context:
         poses = np.zeros(5 * n, np.int32)
         self.ok(self.rt.md_pose_scores(self.h, _f(np.zeros(9 * n)), n, poses.ctypes.data, _f(np.zeros(n))))
 
+    def profile(self, n, t=1):
+        self.ok(self.rt.md_dock_profile(self.h, C.c_void_p(1 << 20), 0, n, t, C.c_void_p(1 << 21), _f(np.zeros(5)),
+                                        None))
+
+    def pose_terms(self, n):
+        tem = np.zeros(3 * n, np.int32)
+        self.ok(self.rt.md_pose_terms(self.h, _f(np.zeros((self.n // 2) ** 3)), _f(np.zeros(9 * n)), n,
+                                      tem.ctypes.data_as(C.POINTER(C.c_int)), _f(np.zeros(9 * n))))
+
+    def adjoint(self, n):
+        poses = np.zeros(5 * n, np.int32)
+        ng3 = (self.n // 2) ** 3
+        self.ok(self.rt.md_adjoint_poses(self.h, _f(np.zeros(9 * n)), n, poses.ctypes.data, _f(np.ones(n)),
+                                         _f(np.zeros(ng3)), _f(np.zeros(ng3)), _f(np.zeros(20)), None, 0, None, None))
+
+    def pairs(self, others, n, t=1):
+        k = len(others)
+        rots, outs = (C.c_void_p * k)(*[1 << 20] * k), (C.c_void_p * k)(*[1 << 21] * k)
+        self.ok(self.rt.md_dock_pairs(self.h, (C.c_void_p * k)(*[o.h.value for o in others]), k, rots,
+                                      (C.c_int * k)(*[n] * k), t, outs))
+
     def capture(self, n, t=1):
         """The launches of md_dock_device on a stream the caller is capturing."""
         first = self.rt.fake_launches()
@@ -148,3 +169,52 @@ def test_uncaptured_work_buffers_do_not_add_up(rt, context):
     before = rt.fake_used()
     b.dock(64)
     assert grown == rt.fake_used() - before
+
+
+# one rotation of the work set at N = 128: 2 x 8 ng N^2 bytes and the charge lists
+ONE_128 = 2 * 8 * 64 * 128 * 128 + 8 * 64 ** 3
+
+
+@pytest.mark.parametrize("call,sets,extra", [
+    (lambda c: c.dock(200), 1, 0),
+    (lambda c: c.dock_device(200), 1, 0),
+    (lambda c: c.profile(200), 1, 0),
+    (lambda c: c.pose_scores(200), 1, 8 * 64 ** 3),
+    (lambda c: c.adjoint(200), 1, 2 * 8 * 64 ** 3),
+    (lambda c: c.pose_terms(200), 1, 201 * 8 * 64 ** 3),   # its own voxel grids: 200 poses
+    (lambda c: c.pairs([c, c], 200), 2, 0),
+])
+def test_automatic_groups_fall_back_to_one_rotation(rt, context, call, sets, extra):
+    """Every call that groups rotations by itself still runs where there is room
+    for one rotation only, does not ask for the large buffers again in later
+    calls, and groups again after md_release_work."""
+    c = context(128)
+    c.ok(rt.md_release_work(c.h))
+    free = rt.fake_used()
+    rt.fake_budget(free + sets * ONE_128 + extra + 4 * MIB)
+    rt.fake_forget()
+    call(c)
+    assert {rt.fake_rotations(k) for k in range(rt.fake_launches())} == {1}
+    refused = rt.fake_refused()
+    call(c)
+    assert rt.fake_refused() == refused
+    rt.fake_budget(1 << 62)
+    c.ok(rt.md_release_work(c.h))
+    rt.fake_forget()
+    call(c)
+    assert max(rt.fake_rotations(k) for k in range(rt.fake_launches())) > 1
+
+
+def test_no_room_for_one_rotation_is_an_error(rt, context):
+    """... after which the same call runs once there is room."""
+    c = context(128)
+    c.ok(rt.md_release_work(c.h))
+    rt.fake_budget(rt.fake_used() + ONE_128 // 2)
+    for call in (c.dock, c.dock_device, c.profile, c.pose_scores, c.pose_terms, lambda n: c.pairs([c], n)):
+        with pytest.raises(AssertionError, match="out of memory"):
+            call(100)
+    rt.fake_budget(1 << 62)
+    for call in (c.dock, c.dock_device, c.profile, c.pose_scores, c.pose_terms, lambda n: c.pairs([c], n)):
+        rt.fake_forget()
+        call(100)
+        assert rt.fake_rotations(0) > 1
