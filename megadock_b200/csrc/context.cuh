@@ -12,6 +12,8 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
+#include <set>
 #include <string>
 #include <tuple>
 #include <vector>
@@ -154,6 +156,27 @@ static_assert(sizeof(md_pose) == sizeof(DevPose), "pose layout");
 
 namespace mdb {
 
+// Runs `set` once for each device (the current one), also when several threads
+// ask at the same time: a kernel's attributes belong to one device's context.
+class OncePerDevice {
+public:
+    template <class Set>
+    cudaError_t run(const Set &set) {
+        int device = 0;
+        cudaError_t e = cudaGetDevice(&device);
+        if (e != cudaSuccess) return e;
+        std::lock_guard<std::mutex> lock(m_);
+        if (done_.count(device)) return cudaSuccess;
+        e = set();
+        if (e == cudaSuccess) done_.insert(device);
+        return e;
+    }
+
+private:
+    std::mutex m_;
+    std::set<int> done_;
+};
+
 // ------------------------------------------------------------------ per-size dispatch
 template <int N>
 struct Sized {
@@ -190,8 +213,10 @@ struct Sized {
     }
 
     static cudaError_t set_attrs() {
-        static bool done = false;
-        if (done) return cudaSuccess;
+        static OncePerDevice once;
+        return once.run(&set_device_attrs);
+    }
+    static cudaError_t set_device_attrs() {
         cudaError_t e = cudaSuccess;
         auto set = [&](const void *f, size_t bytes) {
             if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -209,7 +234,6 @@ struct Sized {
         set((const void *)k_vox_bits<NG, true>, smem_vox());
         set((const void *)k_vox_bits<NG, false>, smem_vox());
         set((const void *)k_xline_fold<N>, xline_smem<N>());
-        if (e == cudaSuccess) done = true;
         return e;
     }
 

@@ -15,7 +15,7 @@ namespace {
 std::map<uintptr_t, size_t> blocks;   // live device blocks: address -> bytes
 uintptr_t next_addr = uintptr_t(1) << 40;
 size_t budget = ~size_t(0), used = 0;
-int refused = 0, device = 0, graphs = 0;
+int refused = 0, device = 0, graphs = 0, attr_calls = 0;
 bool caller_capturing = false;
 cudaError_t last_error = cudaSuccess;
 std::map<int, std::set<const void *>> attrs;   // device -> kernels given their attributes
@@ -29,6 +29,11 @@ size_t fake_used() { return used; }
 int fake_refused() { return refused; }
 void fake_capture(int on) { caller_capturing = on != 0; }
 int fake_graphs() { return graphs; }
+// Attribute calls since the counter was last cleared.
+int fake_attr_calls(int clear) {
+    if (clear) attr_calls = 0;
+    return attr_calls;
+}
 int fake_attrs(int dev) { return (int)attrs[dev].size(); }
 // Bytes of the live block that starts at `addr`; 0 when there is none.
 size_t fake_block(uintptr_t addr) {
@@ -61,6 +66,7 @@ cudaError_t cudaMemcpyAsync(void *dst, const void *, size_t n, cudaMemcpyKind k,
 cudaError_t cudaMemsetAsync(void *, int, size_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute, int) {
     attrs[device].insert(f);
+    ++attr_calls;
     return cudaSuccess;
 }
 cudaError_t cudaLaunchKernel(const void *, dim3, dim3, void **, size_t, cudaStream_t) { return cudaSuccess; }

@@ -218,3 +218,17 @@ def test_no_room_for_one_rotation_is_an_error(rt, context):
         rt.fake_forget()
         call(100)
         assert rt.fake_rotations(0) > 1
+
+
+@pytest.mark.parametrize("n", [48, 128, 256])
+def test_kernel_attributes_are_set_on_every_device(rt, context, n):
+    """The shared-memory opt-in of a size's kernels belongs to one device: a
+    second device's context of that size sets it too, once."""
+    context(n, device=0)
+    before = rt.fake_attrs(1)
+    context(n, device=1)
+    own = rt.fake_attrs(1) - before
+    assert own > 0
+    rt.fake_attr_calls(1)
+    context(n, device=1)
+    assert rt.fake_attr_calls(0) == 0
