@@ -27,8 +27,8 @@ using namespace mdb;
 
 namespace mdb {
 
-// Bound on the candidate groups per rotation of edge N (inv_groups).
-inline size_t cand_groups(size_t N) { return N * kMaxCluster; }
+// Candidate lists per rotation of edge N (inv_groups).
+inline size_t cand_groups(int N);
 
 // Per-launch intermediates for `cap` rotations of one launch group.
 struct WorkSet {
@@ -66,7 +66,7 @@ struct WorkSet {
     static Sizes need(size_t cap, size_t N, size_t t, size_t na) {
         const size_t NG = N / 2;
         return Sizes{{sizeof(float2) * cap * NG * N * N, sizeof(float2) * cap * N * (N / 2) * N,
-                      sizeof(Cand) * cap * cand_groups(N) * t, sizeof(uint32_t) * cap * NG * 2 * NG * ((NG + 31) / 32),
+                      sizeof(Cand) * cap * cand_groups((int)N) * t, sizeof(uint32_t) * cap * NG * 2 * NG * ((NG + 31) / 32),
                       sizeof(int2) * cap * NG * NG * NG, sizeof(int) * cap * NG, sizeof(MarkEntry) * cap * na,
                       sizeof(int) * cap * (NG + 2 * kReach + 1), sizeof(int2) * cap * na, sizeof(int) * cap * (NG + 1),
                       sizeof(uint32_t) * cap * NG * 2 * NG * ((NG + 31) / 32)}};
@@ -316,6 +316,7 @@ namespace mdb {
 // The per-size pipeline entry points of one FFT size.
 struct SizedOps {
     int N;
+    int cand_groups;   // candidate lists per rotation
     cudaError_t (*set_attrs)();
     void (*receptor)(md_ctx *, const float *, const float *);
     void (*voxel_chunk)(md_ctx *, const float *, int, float *, float *);
@@ -325,7 +326,7 @@ struct SizedOps {
 
 template <int N>
 const SizedOps *sized_ops_of() {
-    static const SizedOps ops{N, &Sized<N>::set_attrs, &Sized<N>::receptor, &Sized<N>::voxel_chunk,
+    static const SizedOps ops{N, inv_groups<N>(), &Sized<N>::set_attrs, &Sized<N>::receptor, &Sized<N>::voxel_chunk,
                               &Sized<N>::voxels, &Sized<N>::dock};
     return &ops;
 }
@@ -370,5 +371,7 @@ inline const SizedOps *sized_ops(int N) {
     if (const SizedOps *o = sized_ops_q(N)) return o;
     return sized_ops_r(N);
 }
+
+inline size_t cand_groups(int N) { return sized_ops(N)->cand_groups; }
 
 }  // namespace mdb

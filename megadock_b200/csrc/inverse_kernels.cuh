@@ -260,8 +260,7 @@ constexpr bool inv_plane_owned() {
     return N == 128;
 }
 
-// Candidate groups per rotation of edge N (at most kMaxCluster per plane).
-constexpr int kMaxCluster = 8;
+// Candidate lists per rotation of edge N: one per CTA of each x plane.
 template <int N>
 constexpr int inv_groups() {
     if constexpr (inv_plane_owned<N>()) return N;

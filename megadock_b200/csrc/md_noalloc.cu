@@ -42,7 +42,6 @@ namespace {
 constexpr size_t kScratchBytes = size_t(32) << 20;
 constexpr int kMaxN = 128;
 constexpr int kMaxT = 64;
-constexpr int kMaxNoallocCluster = 2;   // CTAs per plane of the inverse plans up to kMaxN
 constexpr int kMaxDevices = 64;
 // every grid-table size N <= kMaxN
 #define MDB_NOALLOC_SIZES(X)                                                                                  \
@@ -154,7 +153,7 @@ void run_rotation(cudaStream_t s, const LigandView &L, const GridView &G, const 
                                                                  qlist, qcount);
     k_plane_fwd<N, 0><<<dim3(NG, 1), kNT1, Smem<N>::fwd(), s>>>(L, G, vbits, qlist, qcount, nullptr, nullptr, A);
     k_xline_fold<N><<<xline_grid<N>(1), XPlan<N>::NT, Smem<N>::xline(), s>>>(G, A, Rh, Gsp);
-    static_assert(inv_groups<N>() <= N * kMaxNoallocCluster, "candidate scratch");
+    static_assert(inv_groups<N>() == N, "the candidate scratch holds one list per x plane");
     launch_inv<N>(s, G, Gsp, 1, t, 0, cand);
     k_merge<<<1, 256, 0, s>>>(cand, inv_groups<N>(), t, N, nf3f, rot, pose);
 }
@@ -174,7 +173,7 @@ extern "C" int md_dock_noalloc(int nf1, float grid_width, const float *d_grid_co
     auto up = [](size_t b) { return (b + 255) & ~size_t(255); };
     const size_t b_atom = up(sizeof(float4) * na), b_rad = up(sizeof(float2) * na);
     const size_t b_A = up(sizeof(float2) * NG * N * N), b_G = up(sizeof(float2) * N * (N / 2) * N);
-    const size_t b_cand = up(sizeof(Cand) * N * kMaxNoallocCluster * t);
+    const size_t b_cand = up(sizeof(Cand) * N * t);
     const size_t b_bits = up(sizeof(uint32_t) * NG * 2 * NG * ((NG + 31) / 32));
     const size_t b_ql = up(sizeof(int2) * NG * NG * NG), b_qc = up(sizeof(int) * NG);
     const size_t b_sr = up(sizeof(MarkEntry) * na), b_ss = up(sizeof(int) * (NG + 2 * kReach + 1));

@@ -232,3 +232,19 @@ def test_kernel_attributes_are_set_on_every_device(rt, context, n):
     rt.fake_attr_calls(1)
     context(n, device=1)
     assert rt.fake_attr_calls(0) == 0
+
+
+@pytest.mark.parametrize("n,per_plane", [(48, 1), (128, 1), (256, 8)])
+def test_candidate_lists_hold_one_per_cta(rt, context, n, per_plane):
+    """Candidate lists of a launch group: 8 bytes a pose for each CTA that
+    selects (one per x plane up to N = 160, a cluster's CTAs above)."""
+    a, b = context(n, batch=8), context(n, batch=8)
+    for c in (a, b):
+        c.ok(rt.md_set_lanes(c.h, 1))   # one work set
+    before = rt.fake_used()
+    a.dock(8, t=1)
+    one = rt.fake_used() - before
+    before = rt.fake_used()
+    b.dock(8, t=501)
+    poses = 500 * 8 * 20   # the host call's pose records
+    assert rt.fake_used() - before - one == 500 * 8 * 8 * n * per_plane + poses
