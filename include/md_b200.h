@@ -89,9 +89,9 @@ int md_set_batch(md_ctx *ctx, int rotations_per_launch);
  * ones; a graph of the caller's must not be replayed after any of the three. */
 int md_release_work(md_ctx *ctx);
 /* Radix plan of the inverse plane kernel (0, 1 or 2; other values are
- * refused).  At FFT edge 128 it picks the line plans, the kz split reversed or
- * the ky split reversed, and the autotuner (megadock_b200.tune) tries them;
- * every other edge has one measured plan, and the call changes nothing. */
+ * refused).  At FFT edge 128 plan 1 reverses the kz split of plan 0, and the
+ * autotuner (megadock_b200.tune) tries both; 2 is accepted and equals 0.  Every
+ * other edge has one measured plan, and the call changes nothing. */
 int md_set_plan(md_ctx *ctx, int plan);
 /* Tile width asked of the x-line kernel (8, 16 or 32 kz lines; other values
  * are refused).  Every FFT size now runs the one tile shape that measured

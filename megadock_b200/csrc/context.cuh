@@ -118,8 +118,7 @@ struct md_ctx {
     // work sets (lane 0 serves every form; lane 1 the batched graph)
     int batch = 0;   // rotations per launch asked for (md_set_batch); 0 = never asked (group_of)
     int auto_most = kAutoGroup;   // 1 once larger automatic groups had no room (reserve_groups)
-    int plan = 0;   // radix plan variant of the plane top-t kernel (C2RPlan)
-    int tile = 32;  // md_set_tile's value: every size has one x-line shape (XPlan), so it selects nothing
+    int plan = 0;   // md_set_plan's value (inv_forms)
     int lanes = kLanes;   // work sets / capture streams the batched graph alternates over (1 or 2)
     int cap = 0, cap_t = 0, cap_na = 0;
     WorkSet::Sizes have{};           // bytes held by each work-set buffer
@@ -317,6 +316,7 @@ namespace mdb {
 struct SizedOps {
     int N;
     int cand_groups;   // candidate lists per rotation
+    int inv_forms;     // kernels that md_set_plan chooses among
     cudaError_t (*set_attrs)();
     void (*receptor)(md_ctx *, const float *, const float *);
     void (*voxel_chunk)(md_ctx *, const float *, int, float *, float *);
@@ -326,7 +326,7 @@ struct SizedOps {
 
 template <int N>
 const SizedOps *sized_ops_of() {
-    static const SizedOps ops{N, inv_groups<N>(), &Sized<N>::set_attrs, &Sized<N>::receptor, &Sized<N>::voxel_chunk,
+    static const SizedOps ops{N, inv_groups<N>(), inv_forms<N>(), &Sized<N>::set_attrs, &Sized<N>::receptor, &Sized<N>::voxel_chunk,
                               &Sized<N>::voxels, &Sized<N>::dock};
     return &ops;
 }

@@ -260,6 +260,13 @@ constexpr bool inv_plane_owned() {
     return N == 128;
 }
 
+// Forms of the stage that md_set_plan chooses among at edge N; plan 1 is form 1
+// where there are two, every other plan form 0.
+template <int N>
+constexpr int inv_forms() {
+    return inv_plane_owned<N>() ? 2 : 1;
+}
+
 // Candidate lists per rotation of edge N: one per CTA of each x plane.
 template <int N>
 constexpr int inv_groups() {

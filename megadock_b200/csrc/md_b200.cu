@@ -585,21 +585,19 @@ int md_set_lanes(md_ctx *ctx, int lanes) {
     return MD_OK;
 }
 
+// Every size runs the x-line tile that measured fastest for it (XPlan): the
+// value is checked and selects nothing.
 int md_set_tile(md_ctx *ctx, int lines) {
     if (!ctx || (lines != 8 && lines != 16 && lines != 32)) return MD_ERR_ARG;
-    if (lines != ctx->tile) {
-        free_graphs(ctx);
-        ctx->tile = lines;
-    }
     return MD_OK;
 }
 
 int md_set_plan(md_ctx *ctx, int plan) {
     if (!ctx || plan < 0 || plan >= kC2RPlans) return MD_ERR_ARG;
-    if (plan != ctx->plan) {
-        free_graphs(ctx);   // captured launches name the kernels
-        ctx->plan = plan;
-    }
+    // captured launches name the kernels; without a grid nothing is captured
+    const bool forms = ctx->N && sized_ops(ctx->N)->inv_forms > 1;
+    if (forms && (plan == 1) != (ctx->plan == 1)) free_graphs(ctx);
+    ctx->plan = plan;
     return MD_OK;
 }
 

@@ -103,10 +103,18 @@ class FFTProcess:
         self.lanes = int(lanes)
 
     def set_plan(self, plan: int):
-        """Radix plan variant of the inverse plane kernel (0, 1 or 2; they differ
-        at N = 128)."""
+        """Radix plan of the inverse plane kernel (0, 1 or 2; plan_kernel)."""
         _check(N.lib().md_set_plan(self._h, int(plan)), self._h)
         self.plan = int(plan)
+
+    def plan_kernel(self, plan: int) -> int:
+        """The kernel that a plan selects: two at FFT edge 128 (plan 1, the
+        others), one at every other edge."""
+        return int(self.num_fft == 128 and plan == 1)
+
+    def tile_kernel(self, lines: int) -> int:
+        """The kernel that a tile width selects: one per FFT edge."""
+        return 0
 
     # -- FFTProcess::cuda_fft over a rotation range
     def cuda_fft(self, rotmats: np.ndarray, t: int = 1, first_rot: int = 0) -> np.ndarray:

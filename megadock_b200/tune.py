@@ -1,20 +1,19 @@
-"""Autotuner for the batched form: rotations per launch, radix plan and tile.
+"""Autotuner for the batched form: rotations per launch and radix plan.
 
 The batched pipeline's cost per rotation falls as more rotations share a
 launch (fuller grids, fewer launches) until the per-launch intermediates stop
 fitting in L2; at N = 128 the inverse plane kernel has two radix plans
-(md_set_plan), at every other size one measured plan; the x-line kernel has one
-tile shape per size (md_set_tile selects nothing any more, its candidates time
-the same).  ``autotune`` times a sample of rotations with the library's
-per-stage CUDA events (md_dock_profile): first every batch size with plan 0,
-then every plan and tile at the best batch, and keeps the fastest.  Last it
-times the whole
-batched graph (md_dock_device) with one and with two launch groups in flight
-(md_set_lanes): the per-stage events serialise the stages, so they cannot see
-how two groups' kernels share the GPU.  Batch sizes whose two work
-sets would exceed WORK_BUDGET bytes are skipped, and the work buffers are
-released at the end so that the next call allocates them for the chosen
-batch only.  Results are cached per (N, t, sample) in-process.
+(md_set_plan), at every other size one; the x-line kernel has one tile shape
+per size (md_set_tile).  ``autotune`` times a sample of rotations with the
+library's per-stage CUDA events (md_dock_profile): first every batch size with
+the first plan and tile, then, at the best batch, the plans and tiles that
+select another kernel (FFTProcess.plan_kernel, tile_kernel), and keeps the
+fastest.  Last it times the whole batched graph (md_dock_device) with one and
+with two launch groups in flight (md_set_lanes): the per-stage events serialise
+the stages, so they cannot see how two groups' kernels share the GPU.  Batch
+sizes whose two work sets would exceed WORK_BUDGET bytes are skipped, and the
+work buffers are released at the end so that the next call allocates them for
+the chosen batch only.  Results are cached per (N, t, sample) in-process.
 """
 from __future__ import annotations
 
@@ -33,6 +32,17 @@ def work_bytes_per_rotation(n: int) -> int:
     ignored)."""
     ng = n // 2
     return 2 * (8 * ng * n * n + 8 * n * ng * n + 8 * ng ** 3)
+
+
+def _distinct(values, kernel_of):
+    """The values that select different kernels, the first of each; all of them
+    where the context does not say (kernel_of None)."""
+    if kernel_of is None:
+        return list(values)
+    first = {}
+    for v in values:
+        first.setdefault(kernel_of(v), v)
+    return list(first.values())
 
 
 def _time(fp, d_rotmat, d_out, t, sample, b):
@@ -79,14 +89,14 @@ def autotune(fp, d_rotmat: int, d_out: int, t: int, sample: int = 1536, candidat
         if ms < best_ms:
             best_b, best_ms = b, ms
     best_p = plans[0]
-    for p in plans[1:]:
+    for p in _distinct(plans, getattr(fp, "plan_kernel", None))[1:]:
         fp.set_plan(p)
         ms = _time(fp, d_rotmat, d_out, t, sample, best_b)
         if ms < best_ms:
             best_p, best_ms = p, ms
     fp.set_plan(best_p)
     best_t = tiles[0]
-    for tl in tiles[1:]:
+    for tl in _distinct(tiles, getattr(fp, "tile_kernel", None))[1:]:
         fp.set_tile(tl)
         ms = _time(fp, d_rotmat, d_out, t, sample, best_b)
         if ms < best_ms:

@@ -59,3 +59,19 @@ def test_autotune_skips_batches_over_the_work_budget():
     assert 320 * per_rot <= tune.WORK_BUDGET < 384 * per_rot
     b, _ = tune.autotune(fp, 0, 0, 3, sample=256, time_graph=lambda f: 1.0)
     assert b == 320 and fp.released
+
+
+def test_autotune_times_each_kernel_once():
+    """Plans and tiles that a context says select the same kernel are not timed
+    again."""
+    from megadock_b200 import tune
+    from megadock_b200.fft_process import FFTProcess
+
+    class Context(FakeContext):
+        plan_kernel, tile_kernel = FFTProcess.plan_kernel, FFTProcess.tile_kernel
+
+    for n, extra in ((96, 0), (128, 2)):
+        tune._cache.clear()
+        fp = Context(n, best=(32, 0, 32))
+        assert tune.autotune(fp, 0, 0, 3, sample=256, time_graph=lambda f: 1.0) == (32, 0)
+        assert fp.calls == 2 * len(tune.CANDIDATES) + extra and (fp.plan, fp.tile) == (0, 32)

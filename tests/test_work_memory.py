@@ -248,3 +248,20 @@ def test_candidate_lists_hold_one_per_cta(rt, context, n, per_plane):
     b.dock(8, t=501)
     poses = 500 * 8 * 20   # the host call's pose records
     assert rt.fake_used() - before - one == 500 * 8 * 8 * n * per_plane + poses
+
+
+@pytest.mark.parametrize("n,own", [(48, ()), (128, (1,)), (256, ())])
+def test_settings_that_select_no_other_kernel_keep_graphs(rt, context, n, own):
+    """Only a plan with a kernel of its own drops the captured graphs."""
+    c = context(n, batch=4)
+    c.dock(8)
+    graphs = rt.fake_graphs()
+    for tile in (8, 16, 32):
+        c.ok(rt.md_set_tile(c.h, tile))
+    for plan in (2, 1, 2, 0):
+        c.ok(rt.md_set_plan(c.h, plan))
+        if plan not in own:
+            c.dock(8)
+    c.dock(8)
+    assert rt.fake_graphs() == graphs + 1 if own else rt.fake_graphs() == graphs
+    assert rt.md_set_tile(c.h, 12) and rt.md_set_plan(c.h, 3) and rt.md_set_plan(c.h, -1)   # still refused
