@@ -231,7 +231,6 @@ struct Sized {
         if (e == cudaSuccess) e = set_inv_attrs<N>();
         set((const void *)k_xline_rec<N>, smem_xrec());
         set((const void *)k_vox_bits<NG, true>, smem_vox());
-        set((const void *)k_vox_bits<NG, false>, smem_vox());
         set((const void *)k_xline_fold<N>, xline_smem<N>());
         return e;
     }
@@ -279,14 +278,6 @@ struct Sized {
         k_vox_store<NG><<<dim3(NG, nb), kNT0, 0, c->stream>>>(L, w.vbits, w.qlist, w.qcount, d_vr, d_vi);
     }
 
-    static void voxels(md_ctx *c, const float *d_rot9, float *d_vr, float *d_vi) {
-        GridView G{c->ng, c->gw, (float)(c->ng * c->gw) / 2, c->d_gc, c->d_tw};
-        LigandView L{c->na, c->d_atom, c->d_rad2, c->delta};
-        const WorkSet &w = c->ws[0];
-        voxelize(c, w, d_rot9, 1, c->stream);
-        k_vox_store<NG><<<dim3(NG, 1), kNT0, 0, c->stream>>>(L, w.vbits, w.qlist, w.qcount, d_vr, d_vi);
-    }
-
     // One launch group: nb rotations whose matrices start at d_rot9, on work
     // set w and stream s.  With `ev` set, an event is recorded after each of
     // the five stages.
@@ -320,14 +311,18 @@ struct SizedOps {
     cudaError_t (*set_attrs)();
     void (*receptor)(md_ctx *, const float *, const float *);
     void (*voxel_chunk)(md_ctx *, const float *, int, float *, float *);
-    void (*voxels)(md_ctx *, const float *, float *, float *);
     void (*dock)(md_ctx *, const WorkSet &, cudaStream_t, const float *, int, int, int, DevPose *, cudaEvent_t *);
 };
 
 template <int N>
 const SizedOps *sized_ops_of() {
-    static const SizedOps ops{N, inv_groups<N>(), inv_forms<N>(), &Sized<N>::set_attrs, &Sized<N>::receptor, &Sized<N>::voxel_chunk,
-                              &Sized<N>::voxels, &Sized<N>::dock};
+    static const SizedOps ops{N,
+                              inv_groups<N>(),
+                              inv_forms<N>(),
+                              &Sized<N>::set_attrs,
+                              &Sized<N>::receptor,
+                              &Sized<N>::voxel_chunk,
+                              &Sized<N>::dock};
     return &ops;
 }
 

@@ -87,12 +87,6 @@ __device__ __forceinline__ float sqdist(float c, float g) {
     return __fmul_rn(d, d);
 }
 
-template <int NG>
-__device__ __forceinline__ bool vbit(const uint32_t *plane, int q, int s) {
-    constexpr int W = VoxShared<NG>::W;
-    return (plane[q * W + (s >> 5)] >> (s & 31)) & 1u;
-}
-
 // Per-rotation atom record for the voxelizer: rotated coordinates, the
 // search-box origin (src/ligand.cpp:71-73) and both sphere radii squared.
 struct MarkEntry {
@@ -153,8 +147,8 @@ __device__ void vox_mark(VoxShared<NG> &vs, const MarkEntry *__restrict__ rec, i
     __syncthreads();
 }
 
-// Word-parallel form of vox_code: the class bits of 32 cells (row q, word w)
-// of plane p at once.  c2 = "value delta", c1 = "value 1.0".
+// The class bits of 32 cells (row q, word w) of plane p at once: c2 = "value
+// delta" (core), c1 = "value 1.0" (surface).
 template <int NG>
 __device__ __forceinline__ uint32_t vw_core(const VoxShared<NG> &vs, int slot, int q, int w) {
     constexpr int W = VoxShared<NG>::W;
@@ -178,7 +172,9 @@ __device__ __forceinline__ uint32_t vw_inner(int w, int ng) {
     return m;
 }
 
-// core cells of (slot, q, w) that survive the scrape (vox_surv)
+// Core cells of (slot, q, w) that survive the swollen-surface scrape
+// (src/ligand.cpp:110-134): interior cells with a 6-neighbour outside the core
+// lose their core value.
 template <int NG>
 __device__ __forceinline__ uint32_t vw_surv(const VoxShared<NG> &vs, int slot, int i, int q, int w, int ng) {
     const uint32_t c = vw_core<NG>(vs, slot, q, w);
@@ -214,42 +210,6 @@ __device__ __forceinline__ void vox_code_words(const VoxShared<NG> &vs, int p, i
     const uint32_t demote = surv & vw_inner(w, ng) & (es | ez);
     c2 = surv & ~demote;
     c1 |= demote;
-}
-
-// Core bit survives the swollen-surface scrape (src/ligand.cpp:110-134):
-// interior cells with a 6-neighbour outside the core lose their core value.
-template <int NG>
-__device__ __forceinline__ bool vox_surv(const VoxShared<NG> &vs, int slot, int i, int q, int s, int ng) {
-    const uint32_t *c = vs.core[slot];
-    if (!vbit<NG>(c, q, s)) return false;
-    const bool interior = i >= 1 && i <= ng - 2 && q >= 1 && q <= ng - 2 && s >= 1 && s <= ng - 2;
-    if (!interior) return true;
-    return vbit<NG>(vs.core[slot - 1], q, s) && vbit<NG>(vs.core[slot + 1], q, s) && vbit<NG>(c, q - 1, s) &&
-           vbit<NG>(c, q + 1, s) && vbit<NG>(c, q, s - 1) && vbit<NG>(c, q, s + 1);
-}
-
-// Pre-step-4 value class: 2 = core (delta), 1 = surface (1.0), 0 = empty.
-template <int NG>
-__device__ __forceinline__ int vox_class(const VoxShared<NG> &vs, int slot, int i, int q, int s, int ng) {
-    if (vox_surv<NG>(vs, slot, i, q, s, ng)) return 2;
-    return vbit<NG>(vs.surf[slot - 1], q, s) ? 1 : 0;
-}
-
-// Real rPSC class of cell (p, q, s): 2 = core (value delta), 1 = surface
-// (value 1.0), 0 = empty.  With delta != 1 the interior core cells next to an
-// empty cell become surface (src/ligand.cpp:176-195).
-template <int NG>
-__device__ __forceinline__ int vox_code(const VoxShared<NG> &vs, int p, int q, int s, int ng, bool general_delta) {
-    const int c = vox_class<NG>(vs, 2, p, q, s, ng);
-    if (c != 2 || !general_delta) return c;
-    const bool interior = p >= 1 && p <= ng - 2 && q >= 1 && q <= ng - 2 && s >= 1 && s <= ng - 2;
-    if (interior) {
-        if (vox_class<NG>(vs, 1, p - 1, q, s, ng) == 0 || vox_class<NG>(vs, 3, p + 1, q, s, ng) == 0 ||
-            vox_class<NG>(vs, 2, p, q - 1, s, ng) == 0 || vox_class<NG>(vs, 2, p, q + 1, s, ng) == 0 ||
-            vox_class<NG>(vs, 2, p, q, s - 1, ng) == 0 || vox_class<NG>(vs, 2, p, q, s + 1, ng) == 0)
-            return 1;
-    }
-    return 2;
 }
 
 // ------------------------------------------------------------------ atom prep

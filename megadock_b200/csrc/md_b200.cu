@@ -34,8 +34,6 @@ void launch_voxel_chunk(md_ctx *c, const float *rot, int nb, float *vr, float *v
     sized_ops(c->N)->voxel_chunk(c, rot, nb, vr, vi);
 }
 
-void launch_voxels(md_ctx *c, const float *rot, float *vr, float *vi) { sized_ops(c->N)->voxels(c, rot, vr, vi); }
-
 void launch_dock_ws(md_ctx *c, const WorkSet &w, cudaStream_t s, const float *rot, int nb, int rot0, int t,
                     DevPose *pose, cudaEvent_t *ev = nullptr) {
     sized_ops(c->N)->dock(c, w, s, rot, nb, rot0, t, pose, ev);
@@ -1082,7 +1080,7 @@ int md_ligand_voxels(md_ctx *ctx, const float *rotmat9, float *grid_r, float *gr
     float *d_vr = d, *d_vi = d + ng3, *d_rot = d + 2 * ng3;
     cudaError_t e = cudaMemcpyAsync(d_rot, rotmat9, sizeof(float) * 9, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) {
-        launch_voxels(ctx, d_rot, d_vr, d_vi);
+        launch_voxel_chunk(ctx, d_rot, 1, d_vr, d_vi);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(grid_r, d_vr, sizeof(float) * ng3, cudaMemcpyDeviceToHost, ctx->stream);

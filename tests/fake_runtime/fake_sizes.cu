@@ -40,7 +40,6 @@ struct Fake {
     }
     static void receptor(md_ctx *, const float *, const float *) {}
     static void voxel_chunk(md_ctx *c, const float *, int nb, float *, float *) { note(c, c->ws[0], nb, 1); }
-    static void voxels(md_ctx *c, const float *, float *, float *) { note(c, c->ws[0], 1, 1); }
     static void dock(md_ctx *c, const WorkSet &w, cudaStream_t, const float *, int nb, int, int t, DevPose *,
                      cudaEvent_t *) {
         note(c, w, nb, t);
@@ -50,7 +49,6 @@ struct Fake {
             SizedOps x = *sized_ops_of<N>();
             x.receptor = &receptor;
             x.voxel_chunk = &voxel_chunk;
-            x.voxels = &voxels;
             x.dock = &dock;
             return x;
         }();
