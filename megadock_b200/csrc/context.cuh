@@ -294,6 +294,7 @@ struct Sized {
         if (ev) cudaEventRecord(ev[3], s);
         launch_inv<N>(s, G, w.G, nb, t, c->plan, w.cand);
         if (ev) cudaEventRecord(ev[4], s);
+        static_assert(inv_groups<N>() <= kMergeLists, "k_merge's list places");
         k_merge<<<nb, 256, 0, s>>>(w.cand, inv_groups<N>(), t, N, nf3f, rot0, d_pose);
         if (ev) cudaEventRecord(ev[5], s);
     }

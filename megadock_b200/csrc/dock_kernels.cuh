@@ -1696,25 +1696,47 @@ __global__ void __launch_bounds__(kNT, c2r_min_blocks<N, V>())
 }
 
 // ------------------------------------------------------------------ K4
-// Merge the N x t per-plane candidates of one rotation into t pose records
-// with the reference's rules (src/fft_process.cpp:408-458).
-static __global__ void k_merge(const Cand *__restrict__ cand, int nplanes, int t, int N, float nf3f, int rot0,
-                               DevPose *__restrict__ pose) {
+// Merge one rotation's `lists` candidate lists of t into t pose records with
+// the reference's rules (src/fft_process.cpp:408-458).
+//
+// Every list is in selection order (select_cells; a longer one pass after
+// pass), so a round compares the lists' heads only: a thread holds the best
+// head of its lists, and only the round's winner reads again.  Reading all
+// lists x t candidates in each of the t rounds took more time with every list
+// that a cluster's CTAs add, twice the whole call for 100 poses at N = 162 to
+// 224.  100 poses of one rotation, us (B200): N = 160 668 -> 86, 216 3,952 -> 74
+// (880 when a plane had one list), 330 23,974 -> 211; one to ten poses equal up
+// to N = 200, 10 poses of 8 rotations at 512 53 -> 6.7 per rotation.
+constexpr int kMergeLists = 4096;   // N = 512, eight CTAs per plane
+static __global__ void __launch_bounds__(256)
+    k_merge(const Cand *__restrict__ cand, int lists, int t, int N, float nf3f, int rot0, DevPose *__restrict__ pose) {
     __shared__ Cand red[33];
+    __shared__ int pos[kMergeLists];   // place of each list's head; a list belongs to one thread
     const int b = blockIdx.x;
-    const Cand *cb = cand + (size_t)b * nplanes * t;
-    const int n = nplanes * t;
-    Cand prev{0.f, -1};
+    const Cand *cb = cand + (size_t)b * lists * t;
+    for (int g = threadIdx.x; g < lists; g += blockDim.x) pos[g] = 0;
+    int from = 0;   // the list of this thread's best head
+    auto best_head = [&]() {
+        Cand best{0.f, -1};
+#pragma unroll 4
+        for (int g = threadIdx.x; g < lists; g += blockDim.x) {
+            const int p = pos[g];
+            const Cand c = p < t ? cb[(size_t)g * t + p] : Cand{0.f, -1};
+            if (c.idx >= 0 && (best.idx < 0 || key_better(c.key, c.idx, best.key, best.idx))) {
+                best = c;
+                from = g;
+            }
+        }
+        return best;
+    };
+    Cand mine = best_head();
     const int N2 = N * N;
     for (int round = 0; round < t; ++round) {
-        Cand mine{0.f, -1};
-        for (int e = threadIdx.x; e < n; e += blockDim.x) {
-            const Cand c = cb[e];
-            if (c.idx < 0) continue;
-            if (prev.idx >= 0 && !key_better(prev.key, prev.idx, c.key, c.idx)) continue;
-            if (mine.idx < 0 || key_better(c.key, c.idx, mine.key, mine.idx)) mine = c;
+        const Cand prev = block_best(mine, red);
+        if (prev.idx >= 0 && mine.idx == prev.idx) {   // the cells of the lists are distinct
+            ++pos[from];
+            mine = best_head();
         }
-        prev = block_best(mine, red);
         if (threadIdx.x == 0) {
             DevPose r;
             r.rot = rot0 + b;

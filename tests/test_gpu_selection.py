@@ -79,3 +79,43 @@ def test_long_lists_match_fp64(built, gpu, pairs, n):
         assert np.all(np.abs(g["score"] - want) <= RTOL * np.abs(want) + ATOL)
         at = raw[g["i"], g["j"], g["k"]] / float(n) ** 3
         assert np.all(np.abs(g["score"] - at) <= RTOL * np.abs(at) + ATOL)
+
+
+@pytest.mark.parametrize("n", [126, 162, 220, 252])
+@pytest.mark.parametrize("t", [31, 150])
+def test_merged_lists_match_fp64(built, gpu, pairs, n, t):
+    """Lists longer than a pass, merged over 126 to 2,016 of them a rotation
+    (fewer than, and several for each of, the merge's 256 threads)."""
+    from megadock_b200 import rotation_matrices
+    from oracle import oracle as O
+    job, fp = _context(pairs, "-F", str(n))
+    rr, ri = job.receptor_grids()
+    fp.receptor_fft(rr, ri)
+    xyz, rad, q = job.ligand_atoms()
+    m = rotation_matrices(job.rotation_angles()[[123]])
+    got = fp.cuda_fft(m, t=t)
+    gr, gi = O.ligand_grids(O.rotate(xyz, m[0]), rad, q, job.ng1, job.grid_width, job.grid_coord(), job.lig_core)
+    raw = O.raw_scores(O.receptor_spectrum(rr, ri, n, "fp64"), gr, gi, "fp64")
+    want = np.sort(raw.reshape(-1))[::-1][:t] / float(n) ** 3
+    assert np.all(np.abs(got["score"] - want) <= RTOL * np.abs(want) + ATOL)
+    at = raw[got["i"], got["j"], got["k"]] / float(n) ** 3
+    assert np.all(np.abs(got["score"] - at) <= RTOL * np.abs(at) + ATOL)
+    assert len(set(zip(got["i"], got["j"], got["k"]))) == t
+
+
+def test_merge_time_does_not_follow_the_lists(built, gpu, pairs):
+    """A hundred poses of one rotation from 880 lists (N = 220, four CTAs per
+    plane) merge in about the time of 160 lists (N = 160): a round compares the
+    lists' heads.  Scanning every candidate in every round took 4 times as long."""
+    import torch
+
+    from megadock_b200 import rotation_matrices
+    ms = {}
+    for n in (160, 220):
+        job, fp = _context(pairs, "-F", str(n))
+        fp.receptor_fft(*job.receptor_grids())
+        d_rot = torch.from_numpy(np.ascontiguousarray(rotation_matrices(job.rotation_angles()[:1]))).cuda()
+        d_out = torch.zeros(100 * 5, dtype=torch.int32, device="cuda")
+        ms[n] = min(float(fp.dock_profile(d_rot.data_ptr(), 0, 1, 100, d_out.data_ptr())[0][4]) for _ in range(8))
+    print(f"merge of 100 poses: {ms}")
+    assert ms[220] < 2 * ms[160], ms
