@@ -1324,29 +1324,135 @@ __device__ __forceinline__ Cand block_best(Cand mine, Cand *red) {
 // merged instead.  The few threads that hold a score at or above the bound
 // recompute their items (the same bits) and append those cells to a shared
 // list; a cell's rank in the list (equal keys by the lower index) is its place
-// in the output.  A list longer than kSelCap (many equal keys) is found round
-// by round instead, every round rescanning the items for the best cell after
-// the last one.
+// in the output.  When more cells pass the bound than the list holds, the
+// nsel-th best of those it got is a higher bound, and the cells are collected
+// again.  Where that does not end (many equal keys) the cells are found round
+// by round, every round rescanning the items for the best one after the last.
+// Rounds alone, from the first overflow on, took 32 poses at N = 96 7.8 us per
+// rotation instead of 3.8, at 144 25.9 instead of 12.3 and at 160 35 instead of
+// 16 (B200, stage of 32 or 8 rotations per launch).
 constexpr int kSelMax = 32;
 constexpr int kSelLoose = 3;
 constexpr int kSelCap = 256;
+constexpr int kSelRaises = 4;   // times the bound is raised
+
+// What the selection's threads share: the warps' largest lane maxima, then the
+// cells at or above the bound.
+template <int NW>
+struct SelShared {
+    union {
+        float wtop[NW][kSelMax];
+        Cand list[kSelCap];
+    };
+    float thr_w[NW];
+    float thr_all;
+    int nlist;
+    Cand red[33];
+};
+
+// Appends this thread's cells at or above `thr` (after the floor) to the list.
+template <int N, int NT, int COUNT, int Q2, int STEP, class Item, class Shared>
+__device__ __forceinline__ void collect_cells(const Item &item, const Cand &floor, float thr, Shared &sh) {
+#pragma unroll 1
+    for (int it = threadIdx.x; it < COUNT; it += NT) {
+        float2 o[Q2];
+        const int c0 = item(it, o);
+        if (c0 < 0) continue;
+        auto enter = [&](float key, int idx) {
+            if (key >= thr && (floor.idx < 0 || key_better(floor.key, floor.idx, key, idx))) {
+                const int e = atomicAdd(&sh.nlist, 1);
+                if (e < kSelCap) sh.list[e] = Cand{key, idx};
+            }
+        };
+        static_for<0, Q2>([&](auto k2_) {
+            constexpr int k2 = decltype(k2_)::value;
+            enter(o[k2].x, c0 + STEP * k2);
+            enter(o[k2].y, c0 + STEP * k2 + N);
+        });
+    }
+}
+
+// The list's first n entries at their places in selection order.
+template <int NT, class Shared, class Place>
+__device__ __forceinline__ void rank_cells(const Shared &sh, int n, const Place &place) {
+    for (int e = threadIdx.x; e < n; e += NT) {
+        const Cand c = sh.list[e];
+        int rank = 0;
+        for (int f = 0; f < n; ++f) rank += key_better(sh.list[f].key, sh.list[f].idx, c.key, c.idx) ? 1 : 0;
+        place(rank, c);
+    }
+}
+
+// The nsel best of the list's n entries to out.
+template <int NT, class Shared>
+__device__ __forceinline__ void write_cells(const Shared &sh, int n, int nsel, Cand *__restrict__ out) {
+    rank_cells<NT>(sh, n, [&](int rank, const Cand &c) {
+        if (rank < nsel) out[rank] = c;
+    });
+    const int tid = threadIdx.x;
+    if (tid >= n && tid < nsel) out[tid] = Cand{0.f, -1};
+}
+
+// The rest of the selection when the list overflowed at the bound `thr`.  A
+// function of its own: inlined it took registers from the passes before it.
+template <int N, int NT, int COUNT, int Q2, int STEP, class Item, class Shared>
+__device__ __noinline__ void select_overflow(Item item, int nsel, Cand floor, Cand *__restrict__ out, float thr,
+                                             float tmax, Shared *shp) {
+    Shared &sh = *shp;
+    const int tid = threadIdx.x;
+    for (int raise = 0; raise < kSelRaises; ++raise) {
+        rank_cells<NT>(sh, kSelCap, [&](int rank, const Cand &c) {
+            if (rank == nsel - 1) sh.thr_all = c.key;
+        });
+        __syncthreads();
+        const float higher = sh.thr_all;
+        if (!(higher > thr)) break;
+        thr = higher;
+        if (tid == 0) sh.nlist = 0;
+        __syncthreads();
+        if (tmax >= thr) collect_cells<N, NT, COUNT, Q2, STEP>(item, floor, thr, sh);
+        __syncthreads();
+        if (sh.nlist <= kSelCap) {
+            write_cells<NT>(sh, sh.nlist, nsel, out);
+            return;
+        }
+    }
+    Cand prev = floor;
+    for (int r = 0; r < nsel; ++r) {
+        Cand mine{0.f, -1};
+#pragma unroll 1
+        for (int it = tid; it < COUNT; it += NT) {
+            float2 o[Q2];
+            const int c0 = item(it, o);
+            if (c0 < 0) continue;
+            auto look = [&](float key, int idx) {
+                if (key != key || (prev.idx >= 0 && !key_better(prev.key, prev.idx, key, idx))) return;
+                if (mine.idx < 0 || key_better(key, idx, mine.key, mine.idx)) mine = Cand{key, idx};
+            };
+            static_for<0, Q2>([&](auto k2_) {
+                constexpr int k2 = decltype(k2_)::value;
+                look(o[k2].x, c0 + STEP * k2);
+                look(o[k2].y, c0 + STEP * k2 + N);
+            });
+        }
+        prev = block_best(mine, sh.red);
+        if (tid == 0) out[r] = prev.idx >= 0 ? prev : Cand{0.f, -1};
+        if (prev.idx < 0) {
+            for (int r2 = r + 1 + tid; r2 < nsel; r2 += NT) out[r2] = Cand{0.f, -1};
+            break;
+        }
+    }
+}
+
 template <int N, int NT, int COUNT, int Q2, int STEP, bool ALL, class Item>
 __device__ __forceinline__ void select_cells(const Item &item, int nsel, const Cand &floor, Cand *__restrict__ out) {
     static_assert(NT % 32 == 0 && NT <= 1024, "whole warps");
     constexpr int NW = NT / 32;
-    __shared__ float thr_w[NW];
-    __shared__ float thr_all;
-    // the warps' largest lane maxima, then the cells at or above the bound
-    __shared__ union {
-        float wtop[NW][kSelMax];
-        Cand list[kSelCap];
-    } sh;
-    __shared__ int nlist;
-    __shared__ Cand red[33];
+    __shared__ SelShared<NW> sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int TRIPS = (COUNT + NT - 1) / NT;
     const bool fl = floor.idx >= 0;
-    if (tid == 0) nlist = 0;
+    if (tid == 0) sh.nlist = 0;
     float tmax = -INFINITY;   // fmaxf drops NaN keys, which are never selected
     if (!fl) {
 #pragma unroll
@@ -1387,14 +1493,14 @@ __device__ __forceinline__ void select_cells(const Item &item, int nsel, const C
             const unsigned holders = __ballot_sync(0xffffffffu, vo == mo);
             if (lane == __ffs(holders) - 1) v = -INFINITY;
         }
-        if (lane == 0) thr_w[warp] = thw;
+        if (lane == 0) sh.thr_w[warp] = thw;
     }
     __syncthreads();
     float thr;
     if (nsel <= kSelLoose) {
-        thr = thr_w[0];
+        thr = sh.thr_w[0];
 #pragma unroll
-        for (int w = 1; w < NW; ++w) thr = fmaxf(thr, thr_w[w]);
+        for (int w = 1; w < NW; ++w) thr = fmaxf(thr, sh.thr_w[w]);
     } else {
         if (warp == 0) {
             int pos = 0;   // this lane's place in its warp's list
@@ -1406,67 +1512,16 @@ __device__ __forceinline__ void select_cells(const Item &item, int nsel, const C
                 const unsigned holders = __ballot_sync(0xffffffffu, vo == mo);
                 if (lane == __ffs(holders) - 1) ++pos;
             }
-            if (lane == 0) thr_all = best;
+            if (lane == 0) sh.thr_all = best;
         }
         __syncthreads();
-        thr = thr_all;
+        thr = sh.thr_all;
     }
-    if (tmax >= thr) {
-#pragma unroll 1
-        for (int it = tid; it < COUNT; it += NT) {
-            float2 o[Q2];
-            const int c0 = item(it, o);
-            if (c0 < 0) continue;
-            auto enter = [&](float key, int idx) {
-                if (key >= thr && (!fl || key_better(floor.key, floor.idx, key, idx))) {
-                    const int e = atomicAdd(&nlist, 1);
-                    if (e < kSelCap) sh.list[e] = Cand{key, idx};
-                }
-            };
-            static_for<0, Q2>([&](auto k2_) {
-                constexpr int k2 = decltype(k2_)::value;
-                enter(o[k2].x, c0 + STEP * k2);
-                enter(o[k2].y, c0 + STEP * k2 + N);
-            });
-        }
-    }
+    if (tmax >= thr) collect_cells<N, NT, COUNT, Q2, STEP>(item, floor, thr, sh);
     __syncthreads();
-    const int n = nlist;
-    if (n <= kSelCap) {
-        for (int e = tid; e < n; e += NT) {
-            const Cand c = sh.list[e];
-            int rank = 0;
-            for (int f = 0; f < n; ++f) rank += key_better(sh.list[f].key, sh.list[f].idx, c.key, c.idx) ? 1 : 0;
-            if (rank < nsel) out[rank] = c;
-        }
-        if (tid >= n && tid < nsel) out[tid] = Cand{0.f, -1};
-        return;
-    }
-    Cand prev = floor;
-    for (int r = 0; r < nsel; ++r) {
-        Cand mine{0.f, -1};
-#pragma unroll 1
-        for (int it = tid; it < COUNT; it += NT) {
-            float2 o[Q2];
-            const int c0 = item(it, o);
-            if (c0 < 0) continue;
-            auto look = [&](float key, int idx) {
-                if (key != key || (prev.idx >= 0 && !key_better(prev.key, prev.idx, key, idx))) return;
-                if (mine.idx < 0 || key_better(key, idx, mine.key, mine.idx)) mine = Cand{key, idx};
-            };
-            static_for<0, Q2>([&](auto k2_) {
-                constexpr int k2 = decltype(k2_)::value;
-                look(o[k2].x, c0 + STEP * k2);
-                look(o[k2].y, c0 + STEP * k2 + N);
-            });
-        }
-        prev = block_best(mine, red);
-        if (tid == 0) out[r] = prev.idx >= 0 ? prev : Cand{0.f, -1};
-        if (prev.idx < 0) {
-            for (int r2 = r + 1 + tid; r2 < nsel; r2 += NT) out[r2] = Cand{0.f, -1};
-            break;
-        }
-    }
+    const int n = sh.nlist;
+    if (n <= kSelCap) write_cells<NT>(sh, n, nsel, out);
+    else select_overflow<N, NT, COUNT, Q2, STEP>(item, nsel, floor, out, thr, tmax, &sh);
 }
 
 // K3: one x-plane of one rotation.  Input Gh[x][ky < N/2][kz] from
@@ -1683,7 +1738,7 @@ __global__ void __launch_bounds__(kNT, c2r_min_blocks<N, V>())
     }
     const int base = x * N * N;
     select_cells<N, NT, N * Q1, Q2, 2 * Q1 * N, true>(
-        [&](int it, float2(&o)[Q2]) {
+        [=](int it, float2(&o)[Q2]) {
             const int z = it % N, u = it / N;
             static_for<0, Q2>([&](auto n2_) {
                 constexpr int n2 = decltype(n2_)::value;

@@ -182,7 +182,7 @@ __global__ void __cluster_dims__(P::C, 1, 1) __launch_bounds__(P::NT, P::OCC)
     }
     const int base = x * N * N;
     select_cells<N, NT, CB * Q1, Q2, 2 * Q1 * N, N % C == 0>(
-        [&](int it, float2(&o)[Q2]) {
+        [=](int it, float2(&o)[Q2]) {
             const int cc = it % CB, u = it / CB, ccol = rank * CB + cc;
             static_for<0, Q2>([&](auto n2) { o[n2] = S[(u * Q2 + n2) * CB + cc]; });
             Dft<Q2, +1>::run(o);
