@@ -136,9 +136,14 @@ int ensure_work(md_ctx *ctx, int cap, int t, int nsets = 1) {
     return MD_OK;
 }
 
-// Device scratch of the calls outside the docking graph (adjoint, pose
-// scores, pose terms): n sub-buffers of sz[k] bytes, 256-byte aligned, carved
-// from one context buffer that only grows, so repeated calls allocate nothing.
+// Device scratch of the calls outside the docking graph (receptor build,
+// adjoint, pose scores, pose terms, ligand voxels): n sub-buffers of sz[k] bytes,
+// 256-byte aligned, carved from one context buffer that grows to the largest
+// call, so repeated calls allocate nothing.  A buffer made and freed by each
+// call instead took up to 0.7 ms of a 0.1 ms call (one pose's terms at N = 48),
+// whenever no other allocation shared its pages.  md_pose_terms, whose grids
+// grow with its poses, gives a buffer back that it grew above kScratchKept.
+constexpr size_t kScratchKept = size_t(128) << 20;
 int carve_scratch(md_ctx *ctx, const size_t *sz, int n, char **out) {
     size_t off[16], total = 0;
     if (n > 16) return MD_ERR_ARG;
@@ -1005,35 +1010,22 @@ int md_pose_terms(md_ctx *ctx, const float *rec_rpsc, const float *rotmat, int n
     const size_t ng3 = (size_t)ng * ng * ng;
     // poses per launch: their voxel grids within about 1 GB
     const int P = (int)std::max<size_t>(1, std::min<size_t>((size_t)n, ((size_t)1 << 30) / (8 * ng3)));
-    float *d_rot = nullptr, *d_vox = nullptr, *d_terms = nullptr, *d_rpsc = nullptr;
-    int4 *d_tem = nullptr;
-    auto give_back = [&]() {
-        cudaFree(d_rot);
-        cudaFree(d_tem);
-        cudaFree(d_terms);
-        cudaFree(d_rpsc);
-        cudaFree(d_vox);
-        d_rot = d_vox = d_terms = d_rpsc = nullptr;
-        d_tem = nullptr;
-    };
+    const size_t held = ctx->scratch_cap;
+    int B = 1;
+    char *p[5];
+    rc = with_group(ctx, P, B, [&](int) {
+        const size_t sz[5] = {sizeof(float) * 9 * n, sizeof(int4) * n, sizeof(float) * 9 * n, sizeof(float) * ng3,
+                              sizeof(float) * 2 * ng3 * P};
+        return carve_scratch(ctx, sz, 5, p);
+    });
+    if (rc) return rc;
+    float *d_rot = reinterpret_cast<float *>(p[0]), *d_terms = reinterpret_cast<float *>(p[2]);
+    float *d_rpsc = reinterpret_cast<float *>(p[3]), *d_vox = reinterpret_cast<float *>(p[4]);
+    int4 *d_tem = reinterpret_cast<int4 *>(p[1]);
     cudaError_t e = cudaSuccess;
     auto step = [&](cudaError_t x) {
         if (e == cudaSuccess) e = x;
     };
-    int B = 1;
-    rc = with_group(ctx, P, B, [&](int) {
-        e = cudaSuccess;
-        step(cudaMalloc(&d_rot, sizeof(float) * 9 * n));
-        step(cudaMalloc(&d_tem, sizeof(int4) * n));
-        step(cudaMalloc(&d_terms, sizeof(float) * 9 * n));
-        step(cudaMalloc(&d_rpsc, sizeof(float) * ng3));
-        step(cudaMalloc(&d_vox, sizeof(float) * 2 * ng3 * P));
-        if (e == cudaSuccess) return MD_OK;
-        give_back();
-        ctx->err = std::string("pose terms: ") + cudaGetErrorString(e);
-        return MD_ERR_CUDA;
-    });
-    if (rc) return rc;
     std::vector<int4> tem(n);
     for (int p = 0; p < n; ++p) tem[p] = make_int4(tem3[3 * p], tem3[3 * p + 1], tem3[3 * p + 2], 0);
     cudaStream_t s = ctx->stream;
@@ -1057,7 +1049,8 @@ int md_pose_terms(md_ctx *ctx, const float *rec_rpsc, const float *rotmat, int n
         step(cudaMemcpyAsync(terms, d_terms, sizeof(float) * 9 * n, cudaMemcpyDeviceToHost, s));
         step(cudaStreamSynchronize(s));
     }
-    give_back();
+    // a call over hundreds of poses gives its grids back
+    if (ctx->scratch_cap > std::max(held, kScratchKept)) free_scratch(ctx);
     if (e != cudaSuccess) {
         ctx->err = std::string("pose terms: ") + cudaGetErrorString(e);
         return MD_ERR_CUDA;
@@ -1075,9 +1068,10 @@ int md_ligand_voxels(md_ctx *ctx, const float *rotmat9, float *grid_r, float *gr
     int rc = ensure_work(ctx, std::max(1, ctx->batch), 1);
     if (rc) return rc;
     const size_t ng3 = (size_t)ctx->ng * ctx->ng * ctx->ng;
-    float *d = nullptr;
-    MD_CUDA(cudaMalloc(&d, sizeof(float) * (ng3 * 2 + 9)));
-    float *d_vr = d, *d_vi = d + ng3, *d_rot = d + 2 * ng3;
+    const size_t sz[2] = {sizeof(float) * 9, sizeof(float) * 2 * ng3};
+    char *p[2];
+    if ((rc = carve_scratch(ctx, sz, 2, p))) return rc;
+    float *d_rot = reinterpret_cast<float *>(p[0]), *d_vr = reinterpret_cast<float *>(p[1]), *d_vi = d_vr + ng3;
     cudaError_t e = cudaMemcpyAsync(d_rot, rotmat9, sizeof(float) * 9, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) {
         launch_voxel_chunk(ctx, d_rot, 1, d_vr, d_vi);
@@ -1086,7 +1080,6 @@ int md_ligand_voxels(md_ctx *ctx, const float *rotmat9, float *grid_r, float *gr
     if (e == cudaSuccess) e = cudaMemcpyAsync(grid_r, d_vr, sizeof(float) * ng3, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(grid_i, d_vi, sizeof(float) * ng3, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(d);
     if (e != cudaSuccess) {
         ctx->err = std::string("voxelization: ") + cudaGetErrorString(e);
         return MD_ERR_CUDA;

@@ -15,7 +15,7 @@ namespace {
 std::map<uintptr_t, size_t> blocks;   // live device blocks: address -> bytes
 uintptr_t next_addr = uintptr_t(1) << 40;
 size_t budget = ~size_t(0), used = 0;
-int refused = 0, device = 0, graphs = 0, attr_calls = 0;
+int refused = 0, mallocs = 0, device = 0, graphs = 0, attr_calls = 0;
 bool caller_capturing = false;
 cudaError_t last_error = cudaSuccess;
 std::map<int, std::set<const void *>> attrs;   // device -> kernels given their attributes
@@ -27,6 +27,7 @@ extern "C" {
 void fake_budget(size_t bytes) { budget = bytes; }
 size_t fake_used() { return used; }
 int fake_refused() { return refused; }
+int fake_mallocs() { return mallocs; }
 void fake_capture(int on) { caller_capturing = on != 0; }
 int fake_graphs() { return graphs; }
 // Attribute calls since the counter was last cleared.
@@ -42,6 +43,7 @@ size_t fake_block(uintptr_t addr) {
 }
 
 cudaError_t cudaMalloc(void **p, size_t n) {
+    ++mallocs;
     if (used + n > budget) {
         ++refused;
         return last_error = cudaErrorMemoryAllocation;

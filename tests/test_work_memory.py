@@ -265,3 +265,22 @@ def test_settings_that_select_no_other_kernel_keep_graphs(rt, context, n, own):
     c.dock(8)
     assert rt.fake_graphs() == graphs + 1 if own else rt.fake_graphs() == graphs
     assert rt.md_set_tile(c.h, 12) and rt.md_set_plan(c.h, 3) and rt.md_set_plan(c.h, -1)   # still refused
+
+
+@pytest.mark.parametrize("n", [48, 128])
+def test_repeated_small_calls_allocate_nothing(rt, context, n):
+    """The second of two equal calls finds its buffers in place; a call that
+    needed hundreds of MB gives them back."""
+    c = context(n)
+    g = np.zeros((n // 2) ** 3, np.float32)
+    for call in (lambda: c.ok(rt.md_ligand_voxels(c.h, _f(np.zeros(9)), _f(g), _f(g))), lambda: c.pose_terms(3),
+                 lambda: c.pose_scores(3), lambda: c.adjoint(3), lambda: c.dock(3)):
+        call()
+        made = rt.fake_mallocs()
+        call()
+        assert rt.fake_mallocs() == made
+    c.dock(6400)   # the work set at its largest group
+    before = rt.fake_used()
+    many = (200 << 20) // (8 * (n // 2) ** 3)
+    c.pose_terms(many)
+    assert rt.fake_used() <= before
