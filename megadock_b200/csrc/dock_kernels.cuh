@@ -823,7 +823,7 @@ __global__ void __launch_bounds__(FwdPipe<N>::NT, FwdPipe<N>::OCC)
     }
 }
 
-// K1, column-block form (84 < N <= 128, two CTAs per SM, and above 168, where
+// K1, column-block form (84 < N <= 132, two CTAs per SM, and above 168, where
 // the one-CTA form does not fit): the resident z-transformed rows (NG x (N+1))
 // and one N x (CB+1) block buffer: pruned phase 1 from the resident rows into
 // the buffer, phase 2 from the buffer straight to global memory.

@@ -215,7 +215,7 @@ struct InvPlan;
     struct InvPlan<N_> {                                \
         using S = InvSplit<N_, __VA_ARGS__>;            \
     };
-MDB_INV(32, 1, 4, 8, 4, 4, 64, 21) MDB_INV(36, 1, 6, 6, 3, 6, 128, 10) MDB_INV(40, 1, 5, 8, 4, 5, 128, 10)
+MDB_INV(32, 1, 4, 8, 4, 4, 128, 12) MDB_INV(36, 1, 6, 6, 3, 6, 128, 10) MDB_INV(40, 1, 5, 8, 4, 5, 128, 10)
 MDB_INV(42, 1, 6, 7, 3, 7, 192, 7) MDB_INV(44, 1, 4, 11, 2, 11, 288, 5) MDB_INV(48, 1, 6, 8, 4, 6, 160, 8)
 MDB_INV(50, 1, 5, 10, 5, 5, 160, 8) MDB_INV(54, 1, 6, 9, 3, 9, 288, 5) MDB_INV(56, 1, 7, 8, 4, 7, 224, 7)
 MDB_INV(60, 1, 10, 6, 5, 6, 192, 7) MDB_INV(64, 1, 8, 8, 4, 8, 256, 6) MDB_INV(66, 1, 6, 11, 3, 11, 224, 7)
