@@ -466,9 +466,20 @@ __device__ __noinline__ void sum_dense_plane(float *acc, int2 *qs, const int2 *_
     __syncthreads();
 }
 
+// CTAs of k_vox_bits per SM that its shared memory allows (1 KB of each is the
+// system's): eight leave 32 registers a thread, six 40.  The call for dense
+// planes took two registers more than 32 without the bound, 6 % of the
+// voxelizer stage at N = 96 and 126.
+template <int NG>
+constexpr int vox_bits_ctas() {
+    constexpr size_t one = sizeof(VoxShared<NG>) + sizeof(uint32_t) * 2 * NG * VoxShared<NG>::W + sizeof(int2) * kVoxQ + 1040;
+    constexpr int fit = (int)(228 * 1024 / one);
+    return fit >= 8 ? 8 : (fit > 6 ? 6 : fit);
+}
+
 // PREMARKED: the marks come from K0m (marks != nullptr) instead of vox_mark.
 template <int NG, bool PREMARKED = false>
-__global__ void __launch_bounds__(kNT0)
+__global__ void __launch_bounds__(kNT0, vox_bits_ctas<NG>())
     k_vox_bits(LigandView L, GridView G, const MarkEntry *__restrict__ rec, const int *__restrict__ sstart,
                const int2 *__restrict__ cq, const int *__restrict__ cstart, uint32_t *__restrict__ vbits,
                int2 *__restrict__ qlist, int *__restrict__ qcount, const uint32_t *__restrict__ marks = nullptr) {
@@ -1817,11 +1828,12 @@ static __global__ void __launch_bounds__(256)
     const Cand *cb = cand + (size_t)b * lists * t;
     for (int g = threadIdx.x; g < lists; g += blockDim.x) pos[g] = 0;
     int from = 0;   // the list of this thread's best head
-    auto best_head = [&]() {
+    auto best_head = [&](auto at_start) {   // at_start: every list is at its first place
         Cand best{0.f, -1};
 #pragma unroll 4
         for (int g = threadIdx.x; g < lists; g += blockDim.x) {
-            const int p = pos[g];
+            int p = 0;
+            if constexpr (!decltype(at_start)::value) p = pos[g];
             const Cand c = p < t ? cb[(size_t)g * t + p] : Cand{0.f, -1};
             if (c.idx >= 0 && (best.idx < 0 || key_better(c.key, c.idx, best.key, best.idx))) {
                 best = c;
@@ -1830,13 +1842,13 @@ static __global__ void __launch_bounds__(256)
         }
         return best;
     };
-    Cand mine = best_head();
+    Cand mine = best_head(std::true_type{});
     const int N2 = N * N;
     for (int round = 0; round < t; ++round) {
         const Cand prev = block_best(mine, red);
-        if (prev.idx >= 0 && mine.idx == prev.idx) {   // the cells of the lists are distinct
+        if (round + 1 < t && prev.idx >= 0 && mine.idx == prev.idx) {   // the lists' cells are distinct
             ++pos[from];
-            mine = best_head();
+            mine = best_head(std::false_type{});
         }
         if (threadIdx.x == 0) {
             DevPose r;
