@@ -512,7 +512,7 @@ def main():
     ap.add_argument("--plan", type=int, default=0,
                     help="inverse plane kernel radix plan with --batch or --profile-case (0, 1, 2)")
     ap.add_argument("--tile", type=int, default=32,
-                    help="x-line kernel kz lines per CTA with --batch or --profile-case (8, 16, 32)")
+                    help="md_set_tile with --batch or --profile-case (8, 16, 32; selects nothing)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-cufft", action="store_true", help="skip the cuFFT comparator leg")
     ap.add_argument("--workload", default="metric", choices=["metric", "pairs", "adjoint", "fit"],
@@ -521,7 +521,7 @@ def main():
                          "evaluation over 32 planted pairs, 54,000 rotations each")
     ap.add_argument("--fit-pairs", type=int, default=32)
     ap.add_argument("--fft", type=int, default=0, metavar="N",
-                    help="FFT edge of --profile-case (default 128; the bench pair fits every built size)")
+                    help="FFT edge of --profile-case (default 128; the bench pair fits the larger built sizes)")
     ap.add_argument("--profile-case", type=int, default=0, metavar="R",
                     help="run R rotations of the batched form once (for ncu captures) and exit")
     ap.add_argument("--profile-aux", action="store_true",

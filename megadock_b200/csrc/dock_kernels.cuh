@@ -1021,7 +1021,7 @@ __global__ void __launch_bounds__(kNT)
 // pack them.  Output Gh[x][ky][kz], ky < N/2.
 //
 // Bound by instruction issue and the latency of the tile loads (ncu, N = 160:
-// 64 % issue active, 36 % of DRAM peak; N = 256: 41 % and 33 %), so a plan
+// 65 % issue active, 35 % of DRAM peak; N = 256: 45 % and 33 %), so a plan
 // trades radix against warps: F1 near 2 F2 keeps the registers of both passes
 // level, F1 threads per line leave none idle in the two larger passes, and LT
 // = 8 above N = 196 keeps three or more CTAs per SM.  A form that stored the
@@ -1038,7 +1038,8 @@ __global__ void __launch_bounds__(kNT)
 // pair runs out of registers (N = 256 54 -> 47, the older form 50; N = 320 121
 // -> 112; slower by up to 9 % elsewhere).  Four sizes lost to the older form's
 // shorter items (N = 336 136 -> 145, 352 157 -> 173, 384 187 -> 218, 432 364
-// -> 372); every other one gained.
+// -> 372), though no whole call did: with the other stages those edges gained 10,
+// 2, 13 and 1 %; every other one gained here too.
 template <int N>
 struct XPlan;
 #define MDB_XPLAN(N_, F1_, F2_, LT_, OCC_, SEQ_)                               \
@@ -1287,8 +1288,8 @@ __global__ void __launch_bounds__(XPlan<N>::NT, XPlan<N>::OCC)
 // Inverse plane kernels: one thread asks for the rows its CTA's place will need
 // one wave of CTAs later to be brought into L2, so that wave's first loads do
 // not wait for DRAM.  Worth it where a wave of planes (a few hundred, 64 to 200
-// KB each) sits in L2 beside the running one: N = 128 3.31 -> 3.15 us per
-// rotation, 144 5.73 -> 5.51, 160 8.12 -> 7.69, 216 29.8 -> 28.5; 96 and 108
+// KB each) sits in L2 beside the running one: N = 128 3.31 -> 3.21 us per
+// rotation, 144 5.73 -> 5.49, 160 8.12 -> 7.72, 216 29.8 -> 28.4; 96 and 108
 // equal, 256 and 330 1.5 % slower (B200).
 constexpr int kSMs = 148;
 template <int N>

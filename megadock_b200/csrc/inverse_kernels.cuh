@@ -195,7 +195,7 @@ __global__ void __cluster_dims__(P::C, 1, 1) __launch_bounds__(P::NT, P::OCC)
 // The plan of every FFT edge but 128 (k_plane_c2r): MDB_INV(N, C, R1, R2, Q1,
 // Q2, NT, OCC), the fastest measured.
 //
-// Bound by instruction issue (ncu, N = 256: 52 % issue active, 17 % of DRAM
+// Bound by instruction issue (ncu, N = 256: 55 % issue active, 18 % of DRAM
 // peak), then by the cluster barriers and the loads around them.  C is the
 // fewest CTAs that leave room for two or three more clusters on their SMs; a
 // plane that fits one CTA three times over is not split.  Leaving the z
@@ -206,8 +206,9 @@ __global__ void __cluster_dims__(P::C, 1, 1) __launch_bounds__(P::NT, P::OCC)
 // a column launch through global memory above), us per rotation of the stage
 // (B200, one pose): N = 48 0.47 -> 0.27, 96 2.02 -> 1.46, 108 3.09 -> 2.43, 144
 // 6.56 -> 5.8, 160 9.1 -> 8.2, 180 16.6 -> 15.0, 224 28.1 -> 26.5, 256 102 ->
-// 44, 320 150 -> 116, 330 173 -> 138, 512 677 -> 561 (one loses: 192 14.9 ->
-// 15.8); ten poses at N = 126 9.3 -> 5.7.
+// 44, 320 150 -> 116, 330 173 -> 138, 512 677 -> 561 (192 loses, 14.9 -> 15.8,
+// and 450 to 504 up to 17 %; the whole calls there gain 53 and 1 to 18 %); ten
+// poses at N = 126 9.3 -> 5.7.
 template <int N>
 struct InvPlan;
 #define MDB_INV(N_, ...)                               \

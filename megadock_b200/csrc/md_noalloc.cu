@@ -5,9 +5,11 @@
 // that has already reserved all device memory for its own pool allocator, a
 // plugin that must not grow the process's footprint behind its host's back,
 // or a latency-critical loop where cudaMalloc/cudaFree (which synchronise the
-// device) are not allowed.  This entry point runs the same kernels as md_dock
-// but keeps every intermediate in one file-scope static device array, so it
-// calls no cudaMalloc, cudaFree or allocating library routine.  The caller
+// device) are not allowed.  This entry point runs md_dock's kernels (its forward
+// planes always in the one-CTA form, its voxel classes without premarked
+// planes: for one rotation at a time both measure the same) and keeps every
+// intermediate in one file-scope static device array, so it calls no
+// cudaMalloc, cudaFree or allocating library routine.  The caller
 // owns and passes all inputs and outputs as device pointers.
 //
 // Limits and rules:

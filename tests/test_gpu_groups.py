@@ -74,3 +74,37 @@ def test_callers_graph_outlives_larger_calls(built, gpu, pairs, n):
     fp.cuda_fft(mats[:2], t=40)
     assert np.array_equal(replayed(), want)
     assert np.array_equal(fp.cuda_fft(mats[:120], t=2), many)
+
+
+def test_pairs_of_default_contexts(built, gpu, tmp_path):
+    """Pair contexts without a launch size group their rotations too."""
+    import ctypes as C
+
+    import torch
+
+    from megadock_b200 import POSE_DTYPE, FFTProcess, Job, lib, rotation_matrices, synth
+    t, k = 2, 70
+    ctxs, plain = [], []
+    for nr, nl, seed, n in [(30, 16, 8, 64), (60, 40, 32, 84), (30, 16, 9, 180)]:
+        rp, lp = synth.write_pair(str(tmp_path), nr, nl, seed, stem=f"d{seed}")
+        job = Job(["-R", rp, "-L", lp, "-r", "360", "-F", str(n)])
+        mats = rotation_matrices(job.rotation_angles())[:k]
+        for out in (ctxs, plain):
+            fp = FFTProcess(0)
+            fp.alloc_array(job.nf1, job.grid_width, job.grid_coord())
+            job.receptor_to(fp)
+            xyz, rad, q = job.ligand_atoms()
+            fp.ligand_data_transfer_gpu(xyz, rad, q, job.lig_core)
+            out.append(fp)
+    d_rot = torch.from_numpy(np.ascontiguousarray(mats)).cuda()
+    d_out = [torch.zeros(k * t * 5, dtype=torch.int32, device="cuda") for _ in ctxs]
+    torch.cuda.synchronize()
+    runner, m = FFTProcess(0), len(ctxs)
+    rc = lib().md_dock_pairs(runner._h, (C.c_void_p * m)(*[fp._h.value for fp in ctxs]), m,
+                             (C.c_void_p * m)(*[d_rot.data_ptr()] * m), (C.c_int * m)(*[k] * m), t,
+                             (C.c_void_p * m)(*[o.data_ptr() for o in d_out]))
+    assert rc == 0
+    torch.cuda.synchronize()
+    for fp, o in zip(plain, d_out):
+        fp.set_batch(1)
+        assert np.array_equal(o.cpu().numpy().view(POSE_DTYPE), fp.cuda_fft(mats, t=t))
